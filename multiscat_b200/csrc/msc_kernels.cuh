@@ -38,7 +38,8 @@ __host__ __device__ __forceinline__ typename CT<R>::t mk2(R a, R b)
 }
 
 // ---------------------------------------------------------------------------
-// Block-diagonal inverse:  out (=|+=) D^-1 x   on every row of a tile.
+// Block-diagonal inverse on CUDA cores:  out (=|+=) D^-1 x   on every row of a
+// tile (the mixed form's FP32 fallback; FP64 uses k_block_inverse_dmma).
 //   xt = E^T x ; s = sum_k en_k xt_k / (pkd + lam_k) ; beta = c s / (1 - c f_n)
 //   yt = (xt + beta en) / (pkd + lam) ; u = E yt
 // Two GEMMs along z with the tile's 2*TR real columns staged in shared
@@ -181,9 +182,9 @@ k_block_inverse(Tiles tiles, const int *__restrict__ gate, int n, const R *__res
 // ---------------------------------------------------------------------------
 // Residual diagonal part (FP64):  out = b - D x  on every row of a tile.
 //   D x = T x + (Re V00 + pkd) x - c x(z_n) e_n ; b = b_spec e_n on the
-// specular row.  One FP64 GEMM with the symmetric T.  One item per
-// (z, half of the tile's rows); the plan launches 2 n threads (rounded up to
-// a warp) when that is at most 512, so that a block takes one round.
+// specular row.  One FP64 GEMM with the symmetric T, one item per (z, half of
+// the tile's rows).  Used by the allocation-free operator, which has no room
+// for an operand image of T; plans use k_residual_dmma.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(512)
 k_residual_diag(Tiles tiles, const int *__restrict__ gate, int n,

@@ -33,6 +33,7 @@
 
 #include "../../include/multiscat_b200.h"
 #include "msc_common.cuh"
+#include "msc_dmma.cuh"
 #include "msc_eigh.hpp"
 #include "msc_eigh_gpu.cuh"
 #include "msc_kernels.cuh"
@@ -161,9 +162,10 @@ struct msc_plan {
     int R = 0, ntiles = 0;
     std::vector<int> tile_row0_h, tile_nrow_h, tile_sys_h, sys_tile0_h, sys_row0_h, row_sys_h;
     // device data
-    DevBuf<double> E, ET, Tm, lam, en, v00, row_pkd, row_fn;
+    DevBuf<double> E, Tm, lam, en, v00, row_pkd, row_fn;
     DevBuf<double2> Vt, row_c, row_b, row_rhs, sys_aspec;
-    DevBuf<double2> row_cf;        // c / (1 - c f_n) per row (tcgen05 block inverse)
+    DevBuf<double2> row_cf;        // c / (1 - c f_n) per row (tcgen05 and DMMA block inverses)
+    DevBuf<double2> img_et, img_e, img_t;   // DMMA operand images of E^T, E and T
     std::vector<double2> row_c_h, rhs_default_h;   // c per row; default right-hand side
     DevBuf<int> row_pos, pos_map;                  // [R] torus position; [B][nkx*nky] row or -1
     DevBuf<int> sys_row0;                          // [B + 1] first row of each system
@@ -253,9 +255,9 @@ struct msc_plan {
         if (kcyc_host) cudaFreeHost(kcyc_host);
         for (cudaEvent_t e : tev) cudaEventDestroy(e);
         if (stream) cudaStreamDestroy(stream);
-        E.release(); ET.release(); Tm.release(); lam.release(); en.release(); v00.release();
+        E.release(); Tm.release(); lam.release(); en.release(); v00.release();
         row_pkd.release(); row_fn.release(); Vt.release(); row_c.release(); row_b.release();
-        row_cf.release();
+        row_cf.release(); img_et.release(); img_e.release(); img_t.release();
         row_rhs.release(); sys_aspec.release(); row_pos.release(); pos_map.release();
         sys_row0.release(); nbr.release(); tile_row0.release();
         tile_nrow.release(); tile_sys.release(); sys_tile0.release(); sys_spec_row.release();
@@ -326,9 +328,6 @@ cudaError_t refill(DevBuf<T> &buf, const std::vector<T> &h)
 }
 
 int block_inverse_rows(int n) { return n <= msc::kWideNz ? 8 : 4; }
-size_t smem_block_inverse(int n) { return (size_t)2 * n * 2 * block_inverse_rows(n) * sizeof(double); }
-void launch_block_inverse(msc_plan *p, const int *gate, const double2 *x, double2 *out, int acc,
-                          cudaStream_t st);
 size_t smem_residual(int n) { return (size_t)n * 2 * msc::kTileRows * sizeof(double); }
 size_t smem_coupling(int K) { return (size_t)msc::kTileRows * K * sizeof(int); }
 
@@ -340,7 +339,6 @@ struct OpData;   // operator data of one precision
 template <>
 struct OpData<double> {
     static const double *E(msc_plan *p) { return p->E.p; }
-    static const double *ET(msc_plan *p) { return p->ET.p; }
     static const double *lam(msc_plan *p) { return p->lam.p; }
     static const double *en(msc_plan *p) { return p->en.p; }
     static const double *pkd(msc_plan *p) { return p->row_pkd.p; }
@@ -416,40 +414,66 @@ void launch_block_inverse_tc(msc_plan *p, const int *gate, const float2 *x, floa
     }
 }
 
+msc::dm::Params dmma_params(msc_plan *p, const int *gate, const double2 *x, double2 *out, int flag)
+{
+    msc::dm::Params q{};
+    q.n = p->n;
+    q.rows = p->R;
+    q.lam = p->lam.p;
+    q.en = p->en.p;
+    q.row_cf = p->row_cf.p;
+    q.v00 = p->v00.p;
+    q.row_c = p->row_c.p;
+    q.row_rhs = p->row_rhs.p;
+    q.row_pkd = p->row_pkd.p;
+    q.row_sys = p->row_sys.p;
+    q.gate = gate;
+    q.x = x;
+    q.out = out;
+    q.flag = flag;
+    return q;
+}
+
+// out (=|+=) D^-1 x.  FP64: the DMMA kernel (also in place, out = x: a tile is
+// read whole before it is written).
+void launch_block_inverse(msc_plan *p, const int *gate, const double2 *x, double2 *out, int acc,
+                          cudaStream_t st)
+{
+    msc::dm::Params q = dmma_params(p, gate, x, out, acc);
+    q.img1 = p->img_et.p;
+    q.img2 = p->img_e.p;
+    (void)msc::dm::dispatch(true, msc::dm::choose(p->R, p->n), q, st, true);
+}
+
 template <typename R>
 void launch_block_inverse_t(msc_plan *p, const int *gate, const C2<R> *x, C2<R> *out, int acc,
                             cudaStream_t st)
 {
-    using D = OpData<R>;
-    if constexpr (std::is_same<R, float>::value) {
+    if constexpr (std::is_same<R, double>::value) {
+        launch_block_inverse(p, gate, x, out, acc, st);
+    } else {
+        using D = OpData<R>;
         if (p->use_tc && !acc) {
             launch_block_inverse_tc(p, gate, x, out, st);
             return;
         }
+        if (block_inverse_rows(p->n) == 8)
+            msc::k_block_inverse<8, R><<<p->ntiles, 256, smem_block_inverse_t<R>(p->n), st>>>(
+                p->tiles(), gate, p->n, D::E(p), D::ET(p), p->lam.p, p->en.p, p->row_pkd.p,
+                p->row_c.p, p->row_fn.p, x, out, acc);
+        else
+            msc::k_block_inverse<4, R><<<p->ntiles, 256, smem_block_inverse_t<R>(p->n), st>>>(
+                p->tiles(), gate, p->n, D::E(p), D::ET(p), p->lam.p, p->en.p, p->row_pkd.p,
+                p->row_c.p, p->row_fn.p, x, out, acc);
     }
-    if (block_inverse_rows(p->n) == 8)
-        msc::k_block_inverse<8, R><<<p->ntiles, 256, smem_block_inverse_t<R>(p->n), st>>>(
-            p->tiles(), gate, p->n, D::E(p), D::ET(p), p->lam.p, p->en.p, p->row_pkd.p,
-            p->row_c.p, p->row_fn.p, x, out, acc);
-    else
-        msc::k_block_inverse<4, R><<<p->ntiles, 256, smem_block_inverse_t<R>(p->n), st>>>(
-            p->tiles(), gate, p->n, D::E(p), D::ET(p), p->lam.p, p->en.p, p->row_pkd.p,
-            p->row_c.p, p->row_fn.p, x, out, acc);
-}
-
-void launch_block_inverse(msc_plan *p, const int *gate, const double2 *x, double2 *out, int acc,
-                          cudaStream_t st)
-{
-    launch_block_inverse_t<double>(p, gate, x, out, acc, st);
 }
 
 void launch_residual_diag(msc_plan *p, const int *gate, const double2 *x, double2 *out, int with_b,
                           cudaStream_t st)
 {
-    const int nt = 2 * p->n <= 512 ? (2 * p->n + 31) / 32 * 32 : 256;
-    msc::k_residual_diag<<<p->ntiles, nt, smem_residual(p->n), st>>>(
-        p->tiles(), gate, p->n, p->Tm.p, p->v00.p, p->row_pkd.p, p->row_c.p, p->row_rhs.p, x, out,
-        with_b);
+    msc::dm::Params q = dmma_params(p, gate, x, out, with_b);
+    q.img1 = p->img_t.p;
+    (void)msc::dm::dispatch(false, msc::dm::choose(p->R, p->n), q, st, true);
 }
 
 constexpr int kHaloBX = 8;
@@ -965,18 +989,13 @@ msc_status capture(msc_plan *p, void (*rec)(msc_plan *, cudaStream_t), cudaGraph
 
 msc_status set_kernel_attributes(int n, int K)
 {
-    MSC_CUDA(cudaFuncSetAttribute(msc::k_block_inverse<8, double>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem_block_inverse(msc::kWideNz)));
-    MSC_CUDA(cudaFuncSetAttribute(msc::k_block_inverse<4, double>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem_block_inverse(msc::kMaxNz)));
+    MSC_CUDA(msc::dm::set_attributes());
     MSC_CUDA(cudaFuncSetAttribute(msc::k_block_inverse<8, float>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem_block_inverse(msc::kWideNz)));
+                                  (int)smem_block_inverse_t<float>(msc::kWideNz)));
     MSC_CUDA(cudaFuncSetAttribute(msc::k_block_inverse<4, float>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem_block_inverse(msc::kMaxNz)));
+                                  (int)smem_block_inverse_t<float>(msc::kMaxNz)));
     MSC_CUDA(cudaFuncSetAttribute(msc::k_coupling<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)smem_coupling(msc::kMaxTaps)));
 #define MSC_HALO_ATTR(HY, R)                                                                     \
@@ -2212,9 +2231,6 @@ msc_status msc_plan_set_potential(msc_plan *p, const double *potential_values, c
     }
     p->en_host.resize(n);
     for (int k = 0; k < n; ++k) p->en_host[k] = p->E_host[(size_t)(n - 1) * n + k];
-    std::vector<double> ET((size_t)n * n);
-    for (int z = 0; z < n; ++z)
-        for (int k = 0; k < n; ++k) ET[(size_t)k * n + z] = p->E_host[(size_t)z * n + k];
     // coupling taps: every offset d != 0 with V_d or V_{-d} nonzero (the set is
     // closed under d -> -d so that A^H, whose tap at d is conj(V_{-d}), runs on
     // the same offsets and tables)
@@ -2244,11 +2260,22 @@ msc_status msc_plan_set_potential(msc_plan *p, const double *potential_values, c
     for (const double2 &v : p->Vt_host)
         if (!std::isfinite(v.x) || !std::isfinite(v.y)) return fail(MSC_ERR_NONFINITE, "non-finite potential");
     MSC_CUDA(upload(p->E, p->E_host));
-    MSC_CUDA(upload(p->ET, ET));
     MSC_CUDA(upload(p->Tm, p->T_host));
     MSC_CUDA(upload(p->lam, p->lam_host));
     MSC_CUDA(upload(p->en, p->en_host));
     MSC_CUDA(upload(p->v00, p->v00_host));
+    {
+        const size_t ne = msc::dm::image_elems(n);
+        const unsigned nb = (unsigned)std::min<size_t>((ne + 255) / 256, 1024);
+        MSC_CUDA(p->img_et.alloc(ne));
+        MSC_CUDA(p->img_e.alloc(ne));
+        MSC_CUDA(p->img_t.alloc(ne));
+        msc::dm::k_fragment_image<<<nb, 256>>>(n, p->E.p, 1, p->img_et.p);
+        msc::dm::k_fragment_image<<<nb, 256>>>(n, p->E.p, 0, p->img_e.p);
+        // A(z, k) = T[k][z], the element the CUDA-core residual kernel reads
+        msc::dm::k_fragment_image<<<nb, 256>>>(n, p->Tm.p, 1, p->img_t.p);
+        MSC_CUDA(cudaGetLastError());
+    }
     if (p->K > 0) {
         MSC_CUDA(upload(p->Vt, p->Vt_host));
     } else {
@@ -2259,6 +2286,9 @@ msc_status msc_plan_set_potential(msc_plan *p, const double *potential_values, c
         auto to32 = [](const std::vector<double> &v) {
             return std::vector<float>(v.begin(), v.end());
         };
+        std::vector<double> ET((size_t)n * n);
+        for (int z = 0; z < n; ++z)
+            for (int k = 0; k < n; ++k) ET[(size_t)k * n + z] = p->E_host[(size_t)z * n + k];
         MSC_CUDA(upload(p->E32, to32(p->E_host)));
         MSC_CUDA(upload(p->ET32, to32(ET)));
         MSC_CUDA(upload(p->lam32, to32(p->lam_host)));
