@@ -39,6 +39,7 @@
 #include "msc_kernels.cuh"
 #include "msc_tc.cuh"
 #include "msc_tcc.cuh"
+#include "msc_tcs.cuh"
 
 namespace {
 
@@ -201,7 +202,10 @@ struct msc_plan {
     bool use_tc = false;
     int tc_n = 0, tc_tile_rows = 0, tc_ntiles = 0, tc_grid = 0;
     int tc_groups = 1;          // warp groups with their own tile loop (1 or 2), or
-                                // kTcChannelMajor: k_block_inverse_tcc
+                                // kTcChannelMajor: k_block_inverse_tcc, kTcStream:
+                                // k_block_inverse_tcs (E streamed from L2)
+    int tcs_stages[2] = {0, 0};  // ring stages of the streamed form at N = 64, 128 (0: does not fit)
+    DevBuf<__nv_bfloat16> e_img_kz, e_img_zk;   // its operand images
     int tc2_max = 0;            // widest N the two-group kernel may take (0: none)
     size_t tc_smem = 0, tc2_smem = 0;
     bool tcc_ok = false;        // the channel-major kernel fits (E and one A buffer)
@@ -272,7 +276,7 @@ struct msc_plan {
         E32.release(); ET32.release(); lam32.release(); en32.release(); row_pkd32.release();
         row_fn32.release(); Vt32.release(); row_c32.release(); Q32.release(); W32.release();
         T32.release(); T64.release(); X0.release();
-        U32.release(); R64.release(); e_img.release(); tc_error.release(); wait_error.release();
+        U32.release(); R64.release(); e_img.release(); e_img_kz.release(); e_img_zk.release(); tc_error.release(); wait_error.release();
         Hraw.release(); dsum.release(); dcoef.release(); gsave.release();
         gs_sys_lvl.release(); gs_lvl_start.release(); gs_lvl_rows.release();
         gs_low_ptr.release(); gs_low_tap.release(); gs_low_row.release();
@@ -367,6 +371,32 @@ size_t smem_block_inverse_t(int n) { return (size_t)2 * n * 2 * block_inverse_ro
 
 // tc_groups code of the channel-major tcgen05 kernel (k_block_inverse_tcc)
 constexpr int kTcChannelMajor = 3;
+// ... and of the form with E streamed from L2 (k_block_inverse_tcs)
+constexpr int kTcStream = 4;
+
+// One instance of the streamed kernel: its launch, or (attr) its shared-memory limit.
+template <int N, int S>
+cudaError_t tcs_instance(const msc::tc::TcStreamParams &sp, int grid, cudaStream_t st, bool attr)
+{
+    const size_t bytes = msc::tc::stream_smem(sp.t.kp, N, S);
+    if (attr)
+        return cudaFuncSetAttribute(msc::tc::k_block_inverse_tcs<N, S>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    msc::tc::k_block_inverse_tcs<N, S><<<grid, msc::tc::kThreads, bytes, st>>>(sp);
+    return cudaGetLastError();
+}
+
+cudaError_t tcs_dispatch(int N, int S, const msc::tc::TcStreamParams &sp, int grid, cudaStream_t st, bool attr)
+{
+    if (N == 128) {
+        if (S == 4) return tcs_instance<128, 4>(sp, grid, st, attr);
+        if (S == 3) return tcs_instance<128, 3>(sp, grid, st, attr);
+        return tcs_instance<128, 2>(sp, grid, st, attr);
+    }
+    if (S == 4) return tcs_instance<64, 4>(sp, grid, st, attr);
+    if (S == 3) return tcs_instance<64, 3>(sp, grid, st, attr);
+    return tcs_instance<64, 2>(sp, grid, st, attr);
+}
 
 void launch_block_inverse_tc(msc_plan *p, const int *gate, const float2 *x, float2 *out,
                              cudaStream_t st)
@@ -390,6 +420,11 @@ void launch_block_inverse_tc(msc_plan *p, const int *gate, const float2 *x, floa
     prm.error = p->tc_error.p;
     using msc::tc::k_block_inverse_tc;
     constexpr int T = msc::tc::kThreads;
+    if (p->tc_groups == kTcStream) {
+        const msc::tc::TcStreamParams sp{prm, p->e_img_zk.p, p->e_img_kz.p};
+        (void)tcs_dispatch(p->tc_n, p->tcs_stages[p->tc_n == 128], sp, p->tc_grid, st, false);
+        return;
+    }
     if (p->tc_groups == kTcChannelMajor) {
         msc::tc::k_block_inverse_tcc<<<p->tc_grid, T, p->tcc_smem, st>>>(prm);
         return;
@@ -1153,12 +1188,62 @@ size_t tc_request_bytes(int n, int N, int G)
     return std::max(tc_smem_bytes(n, N, G), floor_bytes);
 }
 
+// E too large for shared memory beside a tile (n > 224): the streamed tcgen05
+// form, 32 or 64 channels per tile, as many ring stages (up to 4) as fit.
+msc_status setup_tc_stream(msc_plan *p, int sms, size_t optin)
+{
+    const int n = p->n, kp = (n + 15) / 16 * 16, kb = kp / 8, mt = (n + 127) / 128;
+    cudaFuncAttributes fa{};
+    MSC_CUDA(cudaFuncGetAttributes(&fa, msc::tc::k_block_inverse_tcs<128, 4>));
+    msc::tc::TcStreamParams sp{};
+    sp.t.kp = kp;
+    p->tc_n = 0;
+    for (int w = 0; w < 2; ++w) {
+        const int N = 64 << w;
+        p->tcs_stages[w] = 0;
+        if (mt * N > 512) continue;
+        for (int S = 4; S >= 2 && !p->tcs_stages[w]; --S)
+            if (msc::tc::stream_smem(kp, N, S) + fa.sharedSizeBytes <= optin) p->tcs_stages[w] = S;
+        if (!p->tcs_stages[w]) continue;
+        MSC_CUDA(tcs_dispatch(N, p->tcs_stages[w], sp, 0, nullptr, true));
+        p->tc_n = N;       // the widest that fits; the autotuner times both
+    }
+    if (p->tc_n == 0) return MSC_OK;
+    p->tc_groups = kTcStream;
+    p->tc_tile_rows = p->tc_n / 2;
+    p->tc_ntiles = (p->R + p->tc_tile_rows - 1) / p->tc_tile_rows;
+    p->tc_grid = std::min(p->tc_ntiles, sms);
+    // operand images, one contiguous piece [hi, lo][2 K blocks][M blocks][8 z][8 k]
+    // per 16 of K: K = z for E^T x, K = k for E y
+    std::vector<__nv_bfloat16> zk((size_t)2 * kp * kp, __float2bfloat16(0.f)), kz(zk);
+    const size_t part = (size_t)16 * kp;
+    for (int z = 0; z < n; ++z)
+        for (int k = 0; k < n; ++k) {
+            const double v = p->E_host[(size_t)z * n + k];
+            const __nv_bfloat16 hi = __float2bfloat16_rn((float)v);
+            const __nv_bfloat16 lo = __float2bfloat16_rn((float)(v - (double)__bfloat162float(hi)));
+            const size_t in = (size_t)(z % 8) * 8 + k % 8;
+            const size_t a = (size_t)(z / 16) * 2 * part + ((size_t)(z / 8 % 2) * kb + k / 8) * 64 + in;
+            const size_t b = (size_t)(k / 16) * 2 * part + ((size_t)(k / 8 % 2) * kb + z / 8) * 64 + in;
+            zk[a] = hi;
+            zk[a + part] = lo;
+            kz[b] = hi;
+            kz[b + part] = lo;
+        }
+    MSC_CUDA(upload(p->e_img_zk, zk));
+    MSC_CUDA(upload(p->e_img_kz, kz));
+    MSC_CUDA(p->tc_error.alloc(1));
+    MSC_CUDA(cudaMemset(p->tc_error.p, 0, sizeof(int)));
+    p->use_tc = true;
+    return MSC_OK;
+}
+
 // Decide whether the mixed form uses the tcgen05 block inverse and with what
 // tile width; build the BF16 hi/lo image of E in the kernel's smem order.
 msc_status setup_tensor_core(msc_plan *p)
 {
     p->use_tc = false;
-    if (!p->mixed || (p->desc.flags & 1) || p->n > 256) return MSC_OK;
+    if (!p->mixed || (p->desc.flags & 1) || p->n > msc::tc::kStreamMaxK) return MSC_OK;
     int dev = 0, sms = 0, cc_major = 0, cc_minor = 0, optin = 0;
     MSC_CUDA(cudaGetDevice(&dev));
     MSC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -1168,14 +1253,14 @@ msc_status setup_tensor_core(msc_plan *p)
     if (cc_major != 10 || cc_minor != 0) return MSC_OK;   // tcgen05 path is built for sm_100a
     const int n = p->n;
     int chosen = 0;
-    for (int N = 16; N <= 256; N *= 2) {
+    for (int N = 16; N <= 256 && n <= 256; N *= 2) {
         if (tc_tmem_cols(n, N, 1) > 512) break;
         if (tc_smem_bytes(n, N) + tc_static_for(N) > (size_t)optin) break;
         const int tiles = (p->R + N / 2 - 1) / (N / 2);
         chosen = N;
         if (tiles <= sms) break;   // enough tiles for every SM already at this width
     }
-    if (chosen == 0) return MSC_OK;
+    if (chosen == 0) return setup_tc_stream(p, sms, (size_t)optin);
     p->tc_n = chosen;
     p->tc_groups = 1;
     p->tc_tile_rows = chosen / 2;
@@ -1282,6 +1367,13 @@ void apply_tc_width(msc_plan *p, int N, int G = 1)
     int sms = 148, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (p->tc_groups == kTcStream) {           // n > 224: the only form that fits
+        p->tc_n = N >= 128 && p->tcs_stages[1] ? 128 : p->tcs_stages[0] ? 64 : 128;
+        p->tc_tile_rows = p->tc_n / 2;
+        p->tc_ntiles = (p->R + p->tc_tile_rows - 1) / p->tc_tile_rows;
+        p->tc_grid = std::min(p->tc_ntiles, sms);
+        return;
+    }
     if (G == kTcChannelMajor) {
         if (p->tcc_ok) {
             p->tc_n = 128;                 // M rows: 64 channels
@@ -1402,6 +1494,7 @@ msc_status autotune_measure(msc_plan *p)
             p->halo32 = best_k;
         }
         if (p->use_tc) {
+            const bool stream = p->tc_groups == kTcStream;
             const int best_n0 = p->tc_n;
             int best_n = 0, best_g = 1;
             float best_t = 0.f;
@@ -1414,13 +1507,15 @@ msc_status autotune_measure(msc_plan *p)
             // (the channel-major form, MSC_TUNE bg=3, is left out: 243 against
             // 250 us per full-batch launch on the 512-beam cfg2 batch, but the
             // batch was not faster end to end with it)
-            for (int G = 1; G <= 2; ++G)
-                for (int N = 16; N <= (G == 1 ? best_n0 : p->tc2_max); N *= 2) {
+            for (int G = 1; G <= (stream ? 1 : 2); ++G)
+                for (int N = stream ? 64 : 16; N <= (G == 1 ? best_n0 : p->tc2_max); N *= 2) {
                     apply_tc_width(p, N, G);
+                    if (stream && p->tc_n != N) continue;    // does not fit at this width
                     const float t = time_launch(p, [&](cudaStream_t st) {
                         launch_block_inverse_t<float>(p, nullptr, a, b, 0, st);
                     });
-                    p->tune_log.push_back({std::string("block_inverse32_tc") + (G == 2 ? "2" : "") +
+                    p->tune_log.push_back({std::string("block_inverse32_tc") +
+                                               (stream ? "_stream" : G == 2 ? "2" : "") +
                                                "_N" + std::to_string(N) + "_us",
                                            t});
                     if (best_n == 0 || t < best_t) {
@@ -2625,6 +2720,7 @@ const char *msc_plan_tuning_report(msc_plan *p)
          ",coupling32=" + std::string(p->use_halo ? kn[p->halo32] : kn[0]) +
          ",block_inverse32=" + (!p->use_tc ? std::string("simt")
                                 : p->tc_groups == kTcChannelMajor ? std::string("tcc")
+                                : p->tc_groups == kTcStream ? "tc_stream_N" + std::to_string(p->tc_n)
                                 : std::string(p->tc_groups == 2 ? "tc2_N" : "tc_N") + std::to_string(p->tc_n)) +
          "\", \"arnoldi_stream\": \"" + (p->mixed && p->dcgs && p->bulk_arnoldi > 0 ? (p->bulk_arnoldi > 1 ? "bulk" : "bulk_reduce") : "registers") +
          "\"}";
