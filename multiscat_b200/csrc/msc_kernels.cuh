@@ -693,376 +693,6 @@ k_coupling_halo(CouplingTiles ct, const int *__restrict__ gate, int n,
 }
 
 // ---------------------------------------------------------------------------
-// Channel coupling of a separable potential: when every z's tap window
-// factorises as V_(sdx, sdy)(z) = p_sdx(z) q_sdy(z) off the centre (the
-// corrugated Morse potential of a square lattice, xi = (h/2)(cos X + cos Y),
-// gives exactly that: the FFT of e^{2 alpha xi} is a product of two 1-D
-// transforms), the 2-D convolution is a pass along x and a pass along y:
-//   t(x, y')  = sum_sdx p_sdx src(x - sdx, y')            (y' over the halo)
-//   out(x, y) = in0 + sgn [sum_sdy q_sdy t(x, y - sdy) - kappa src(x, y)]
-// with kappa = p_0 q_0 the product's value at the centre, which is no tap.
-// (2 HX + 1) (8 + 2 HY) + 8 (2 HY + 2) complex MACs per thread for 8
-// outputs instead of 8 K: 28 instead of 80 per output for |m|,|n| <= 4, 43
-// instead of 288 for |m|,|n| <= 8.  A thread owns one (x, z) column of the
-// 8 x 8 patch: pass 1 keeps the column's 8 + 2 HY values of t in registers,
-// pass 2 reads nothing but its own registers and the q row.  The halo of the
-// patch is staged as in k_coupling_halo.
-// ---------------------------------------------------------------------------
-struct SepTaps {
-    const void *p;       // [2 HX + 1][n] complex (R), p_sdx at sdx + HX
-    const void *q;       // [2 HY + 1][n] complex (R), q_sdy at sdy + HY
-    const void *kappa;   // [n] complex (R)
-};
-
-// (Staging the halo by one bulk copy per halo position instead, on an
-// mbarrier, measured the same: 283 against 280 us on the 512-beam batch.)
-// HXT > 0 fixes the x reach at compile time (square windows: HXT = HY), so
-// the x pass over the 2 HX + 1 halo columns unrolls; 0 takes it from ct.hx.
-template <int HY, int BX, int ZC, typename R, int HXT = 0>
-__global__ void __launch_bounds__(BX * ZC, HY <= 4 ? 3 : 1)
-k_coupling_sep(CouplingTiles ct, const int *__restrict__ gate, int n, SepTaps sep,
-               const typename CT<R>::t *__restrict__ src, const typename CT<R>::t *__restrict__ in0,
-               R sgn, typename CT<R>::t *__restrict__ out)
-{
-    using C2 = typename CT<R>::t;
-    constexpr int BY = 8;
-    constexpr int HYW = BY + 2 * HY;
-    constexpr int WY = 2 * HY + 1;
-    constexpr int NT = BX * ZC;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int HX = HXT > 0 ? HXT : ct.hx;
-    const int HXW = BX + 2 * HX;
-    const int WX = 2 * HX + 1;
-    C2 *halo = reinterpret_cast<C2 *>(smem_raw);                       // [HXW][HYW][ZC]
-    C2 *pw = halo + (size_t)HXW * HYW * ZC;                            // [WX][ZC]
-    C2 *qw = pw + (size_t)WX * ZC;                                     // [WY][ZC]
-    C2 *kw = qw + (size_t)WY * ZC;                                     // [ZC]
-    int *rows = reinterpret_cast<int *>(kw + ZC);                      // [HXW][HYW]
-
-    const int w = blockIdx.x;
-    const int s = ct.work[3 * w];
-    if (gate && gate[s] == 0) return;
-    const int x0 = ct.work[3 * w + 1], y0 = ct.work[3 * w + 2];
-    const int z0 = blockIdx.y * ZC;
-    const int nkx = ct.nkx, nky = ct.nky;
-    const int *pr = ct.pos_row + (size_t)s * nkx * nky;
-    const C2 *P = reinterpret_cast<const C2 *>(sep.p);
-    const C2 *Qv = reinterpret_cast<const C2 *>(sep.q);
-    const C2 *Kp = reinterpret_cast<const C2 *>(sep.kappa);
-    for (int i = threadIdx.x; i < (WX + WY + 1) * ZC; i += NT) {
-        const int row = i / ZC, z = z0 + (i % ZC);
-        C2 v = mk2<R>(0, 0);
-        if (z < n) v = row < WX ? P[(size_t)row * n + z]
-                     : row < WX + WY ? Qv[(size_t)(row - WX) * n + z] : Kp[z];
-        pw[i] = v;          // pw, qw and kw are consecutive
-    }
-    const int npos = HXW * HYW;
-    for (int pidx = threadIdx.x; pidx < npos; pidx += NT) {
-        const int hy = pidx % HYW, hx = pidx / HYW;
-        int gx = (x0 + hx - HX) % nkx;
-        if (gx < 0) gx += nkx;
-        int gy = (y0 + hy - HY) % nky;
-        if (gy < 0) gy += nky;
-        rows[pidx] = pr[gx * nky + gy];
-    }
-    __syncthreads();
-    const int total = npos * ZC;
-    constexpr int kU = 8;
-    if (std::is_same<R, float>::value && (n % 2) == 0) {
-        const int total2 = total / 2;
-        float4 *halo4 = reinterpret_cast<float4 *>(halo);
-        for (int base = threadIdx.x; base < total2; base += NT * kU) {
-            float4 v[kU];
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int idx = base + u * NT;
-                v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (idx < total2) {
-                    const int row = rows[(2 * idx) / ZC];
-                    const int z = z0 + ((2 * idx) % ZC);
-                    if (row >= 0 && z < n)
-                        v[u] = *reinterpret_cast<const float4 *>(src + (size_t)row * n + z);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int idx = base + u * NT;
-                if (idx < total2) halo4[idx] = v[u];
-            }
-        }
-    } else {
-        for (int base = threadIdx.x; base < total; base += NT * kU) {
-            C2 v[kU];
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int idx = base + u * NT;
-                v[u] = mk2<R>(0, 0);
-                if (idx < total) {
-                    const int row = rows[idx / ZC];
-                    const int z = z0 + (idx % ZC);
-                    if (row >= 0 && z < n) v[u] = src[(size_t)row * n + z];
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int idx = base + u * NT;
-                if (idx < total) halo[idx] = v[u];
-            }
-        }
-    }
-    __syncthreads();
-
-    const int zl = threadIdx.x % ZC;
-    const int tx = threadIdx.x / ZC;
-    const int z = z0 + zl;
-    bool any = false;       // a channel in this patch column (staged rows table)
-#pragma unroll
-    for (int y = 0; y < BY; ++y) any |= (y0 + y < nky) && rows[(tx + HX) * HYW + y + HY] >= 0;
-    if (x0 + tx >= nkx || z >= n || !any) return;
-    // pass 1: t(hy) = sum_sdx p_sdx halo(tx - sdx + HX, hy) over the halo column
-    R tr[HYW], ti[HYW];
-#pragma unroll
-    for (int i = 0; i < HYW; ++i) {
-        tr[i] = 0;
-        ti[i] = 0;
-    }
-#pragma unroll
-    for (int sdx = -HX; sdx <= HX; ++sdx) {
-        const C2 pv = pw[(sdx + HX) * ZC + zl];
-        const C2 *colp = halo + (size_t)(tx - sdx + HX) * HYW * ZC + zl;
-#pragma unroll
-        for (int i = 0; i < HYW; ++i) {
-            const C2 v = colp[(size_t)i * ZC];
-            tr[i] = fma(pv.x, v.x, fma(-pv.y, v.y, tr[i]));
-            ti[i] = fma(pv.x, v.y, fma(pv.y, v.x, ti[i]));
-        }
-    }
-    // pass 2: out(y) = sum_sdy q_sdy t(y - sdy + HY) - kappa src(x, y)
-    C2 qv[WY];
-#pragma unroll
-    for (int i = 0; i < WY; ++i) qv[i] = qw[i * ZC + zl];
-    const C2 kap = kw[zl];
-    const C2 *own = halo + (size_t)(tx + HX) * HYW * ZC + zl;
-    // the patch column's rows come from the staged rows table (its interior
-    // positions), and the in0 values of all BY outputs are loaded before the
-    // arithmetic: no global load waits on another inside the output loop
-    int rowv[BY];
-    C2 base[BY];
-#pragma unroll
-    for (int y = 0; y < BY; ++y)
-        rowv[y] = (y0 + y < nky) ? rows[(tx + HX) * HYW + y + HY] : -1;
-#pragma unroll
-    for (int y = 0; y < BY; ++y)
-        base[y] = (in0 && rowv[y] >= 0) ? in0[(size_t)rowv[y] * n + z] : mk2<R>(0, 0);
-#pragma unroll
-    for (int y = 0; y < BY; ++y) {
-        if (rowv[y] < 0) continue;
-        const C2 c = own[(size_t)(y + HY) * ZC];
-        R ar = -(kap.x * c.x - kap.y * c.y), ai = -(kap.x * c.y + kap.y * c.x);
-#pragma unroll
-        for (int sdy = -HY; sdy <= HY; ++sdy) {
-            const C2 q = qv[sdy + HY];
-            const R xr = tr[y - sdy + HY], xi = ti[y - sdy + HY];
-            ar = fma(q.x, xr, fma(-q.y, xi, ar));
-            ai = fma(q.x, xi, fma(q.y, xr, ai));
-        }
-        out[(size_t)rowv[y] * n + z] = mk2<R>(base[y].x + sgn * ar, base[y].y + sgn * ai);
-    }
-}
-
-// The separable coupling with the x pass run along the halo rows: one
-// thread per (halo row, z) holds the row's BX + 2 HX values in registers
-// and writes the BX values of t over the row's middle columns; the y pass
-// then runs per (x, z) column as in k_coupling_sep.  Each halo value is read
-// from shared memory once by the x pass instead of by up to 2 HX + 1
-// threads: about half the shared-memory operations of k_coupling_sep, whose
-// x pass is bound by them.  With 2 HX >= BX the row's t values go to its
-// 2 HX outer columns (already read), so the patch's own values stay for
-// the kappa term; narrower windows write t over the patch columns and keep
-// the own values in registers.  The x reach HXT is a template parameter
-// (the row lives in registers); the plan runs this form only for windows
-// with hx = HXT.
-template <int HY, int BX, int ZC, typename R, int HXT>
-__global__ void __launch_bounds__(BX * ZC, HY <= 4 ? 3 : 1)
-k_coupling_sep_rows(CouplingTiles ct, const int *__restrict__ gate, int n, SepTaps sep,
-                    const typename CT<R>::t *__restrict__ src,
-                    const typename CT<R>::t *__restrict__ in0, R sgn,
-                    typename CT<R>::t *__restrict__ out)
-{
-    using C2 = typename CT<R>::t;
-    constexpr int BY = 8;
-    constexpr int HYW = BY + 2 * HY;
-    constexpr int WY = 2 * HY + 1;
-    constexpr int NT = BX * ZC;
-    constexpr int HX = HXT;
-    constexpr int HXW = BX + 2 * HX;
-    constexpr int WX = 2 * HX + 1;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    C2 *halo = reinterpret_cast<C2 *>(smem_raw);                       // [HXW][HYW][ZC]
-    C2 *pw = halo + (size_t)HXW * HYW * ZC;                            // [WX][ZC]
-    C2 *qw = pw + (size_t)WX * ZC;                                     // [WY][ZC]
-    C2 *kw = qw + (size_t)WY * ZC;                                     // [ZC]
-    int *rows = reinterpret_cast<int *>(kw + ZC);                      // [HXW][HYW]
-
-    const int w = blockIdx.x;
-    const int s = ct.work[3 * w];
-    if (gate && gate[s] == 0) return;
-    const int x0 = ct.work[3 * w + 1], y0 = ct.work[3 * w + 2];
-    const int z0 = blockIdx.y * ZC;
-    const int nkx = ct.nkx, nky = ct.nky;
-    const int *pr = ct.pos_row + (size_t)s * nkx * nky;
-    const C2 *P = reinterpret_cast<const C2 *>(sep.p);
-    const C2 *Qv = reinterpret_cast<const C2 *>(sep.q);
-    const C2 *Kp = reinterpret_cast<const C2 *>(sep.kappa);
-    for (int i = threadIdx.x; i < (WX + WY + 1) * ZC; i += NT) {
-        const int row = i / ZC, z = z0 + (i % ZC);
-        C2 v = mk2<R>(0, 0);
-        if (z < n) v = row < WX ? P[(size_t)row * n + z]
-                     : row < WX + WY ? Qv[(size_t)(row - WX) * n + z] : Kp[z];
-        pw[i] = v;          // pw, qw and kw are consecutive
-    }
-    constexpr int npos = HXW * HYW;
-    for (int pidx = threadIdx.x; pidx < npos; pidx += NT) {
-        const int hy = pidx % HYW, hx = pidx / HYW;
-        int gx = (x0 + hx - HX) % nkx;
-        if (gx < 0) gx += nkx;
-        int gy = (y0 + hy - HY) % nky;
-        if (gy < 0) gy += nky;
-        rows[pidx] = pr[gx * nky + gy];
-    }
-    __syncthreads();
-    constexpr int kU = 8;
-    constexpr int total = npos * ZC;
-    if (std::is_same<R, float>::value && (n % 2) == 0) {
-        constexpr int total2 = total / 2;
-        float4 *halo4 = reinterpret_cast<float4 *>(halo);
-        for (int base = threadIdx.x; base < total2; base += NT * kU) {
-            float4 v[kU];
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int idx = base + u * NT;
-                v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (idx < total2) {
-                    const int row = rows[(2 * idx) / ZC];
-                    const int z = z0 + ((2 * idx) % ZC);
-                    if (row >= 0 && z < n)
-                        v[u] = *reinterpret_cast<const float4 *>(src + (size_t)row * n + z);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int idx = base + u * NT;
-                if (idx < total2) halo4[idx] = v[u];
-            }
-        }
-    } else {
-        for (int base = threadIdx.x; base < total; base += NT * kU) {
-            C2 v[kU];
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int idx = base + u * NT;
-                v[u] = mk2<R>(0, 0);
-                if (idx < total) {
-                    const int row = rows[idx / ZC];
-                    const int z = z0 + (idx % ZC);
-                    if (row >= 0 && z < n) v[u] = src[(size_t)row * n + z];
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int idx = base + u * NT;
-                if (idx < total) halo[idx] = v[u];
-            }
-        }
-    }
-    __syncthreads();
-
-    // t(x) goes to column tcol(x): the outer columns x < HX and
-    // HX + BX .. HX + BX + (BX - HX) - 1 when they are enough, else over
-    // the patch columns HX + x
-    constexpr bool kOuter = 2 * HX >= BX;
-    auto tcol = [](int x) { return kOuter ? (x < HX ? x : x + BX) : x + HX; };
-    const int zl = threadIdx.x % ZC;
-    const int tx = threadIdx.x / ZC;
-    const C2 *own = halo + (size_t)(tx + HX) * HYW * ZC + zl;
-    C2 cen[kOuter ? 1 : BY];
-    if constexpr (!kOuter) {
-        // the column's own values (kappa term), before the x pass overwrites them
-#pragma unroll
-        for (int y = 0; y < BY; ++y) cen[y] = own[(size_t)(y + HY) * ZC];
-        __syncthreads();
-    }
-
-    // x pass, one thread per halo row (hy, z): t(x, hy) = sum_sdx p_sdx
-    // src(x - sdx, hy) for the patch's BX columns, written to columns
-    // tcol(x) of the same row (no other thread touches that row)
-    for (int item = threadIdx.x; item < HYW * ZC; item += NT) {
-        const int hy = item / ZC, zr = item - hy * ZC;
-        C2 *rowp = halo + (size_t)hy * ZC + zr;          // element hx at rowp[hx * HYW * ZC]
-        C2 pv[WX], rv[HXW];
-#pragma unroll
-        for (int i = 0; i < WX; ++i) pv[i] = pw[i * ZC + zr];
-#pragma unroll
-        for (int i = 0; i < HXW; ++i) rv[i] = rowp[(size_t)i * HYW * ZC];
-#pragma unroll
-        for (int x = 0; x < BX; ++x) {
-            R ar = 0, ai = 0;
-#pragma unroll
-            for (int sdx = -HX; sdx <= HX; ++sdx) {
-                const C2 v = rv[x - sdx + HX];
-                const C2 q = pv[sdx + HX];
-                ar = fma(q.x, v.x, fma(-q.y, v.y, ar));
-                ai = fma(q.x, v.y, fma(q.y, v.x, ai));
-            }
-            rowp[(size_t)tcol(x) * HYW * ZC] = mk2<R>(ar, ai);
-        }
-    }
-    __syncthreads();
-
-    // y pass, one thread per patch column (x, z): out(y) = in0 + sgn
-    // [sum_sdy q_sdy t(x, y - sdy) - kappa src(x, y)]
-    const int z = z0 + zl;
-    bool any = false;       // a channel in this patch column (staged rows table)
-#pragma unroll
-    for (int y = 0; y < BY; ++y) any |= (y0 + y < nky) && rows[(tx + HX) * HYW + y + HY] >= 0;
-    if (x0 + tx >= nkx || z >= n || !any) return;
-    const C2 *tcolp = halo + (size_t)tcol(tx) * HYW * ZC + zl;
-    R tr[HYW], ti[HYW];
-#pragma unroll
-    for (int i = 0; i < HYW; ++i) {
-        const C2 v = tcolp[(size_t)i * ZC];
-        tr[i] = v.x;
-        ti[i] = v.y;
-    }
-    C2 qv[WY];
-#pragma unroll
-    for (int i = 0; i < WY; ++i) qv[i] = qw[i * ZC + zl];
-    const C2 kap = kw[zl];
-    int rowv[BY];
-    C2 base[BY];
-#pragma unroll
-    for (int y = 0; y < BY; ++y)
-        rowv[y] = (y0 + y < nky) ? rows[(tx + HX) * HYW + y + HY] : -1;
-#pragma unroll
-    for (int y = 0; y < BY; ++y)
-        base[y] = (in0 && rowv[y] >= 0) ? in0[(size_t)rowv[y] * n + z] : mk2<R>(0, 0);
-#pragma unroll
-    for (int y = 0; y < BY; ++y) {
-        if (rowv[y] < 0) continue;
-        const C2 c = kOuter ? own[(size_t)(y + HY) * ZC] : cen[kOuter ? 0 : y];
-        R ar = -(kap.x * c.x - kap.y * c.y), ai = -(kap.x * c.y + kap.y * c.x);
-#pragma unroll
-        for (int sdy = -HY; sdy <= HY; ++sdy) {
-            const C2 q = qv[sdy + HY];
-            const R xr = tr[y - sdy + HY], xi = ti[y - sdy + HY];
-            ar = fma(q.x, xr, fma(-q.y, xi, ar));
-            ai = fma(q.x, xi, fma(q.y, xr, ai));
-        }
-        out[(size_t)rowv[y] * n + z] = mk2<R>(base[y].x + sgn * ar, base[y].y + sgn * ai);
-    }
-}
-
-// ---------------------------------------------------------------------------
 // Arnoldi reductions.  partial[tile][i] = sum conj(Q_i) W over the tile for
 // i < nvec; slot nvec holds ||W||^2 when with_norm.  One warp per vector;
 // FP64 accumulation for both precisions.

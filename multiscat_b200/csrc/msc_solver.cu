@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "../../include/multiscat_b200.h"
+#include "msc_box.cuh"
 #include "msc_common.cuh"
 #include "msc_dmma.cuh"
 #include "msc_eigh.hpp"
@@ -223,9 +224,17 @@ struct msc_plan {
     bool use_halo = false;             // halo tables built (taps reach <= 8)
     int halo32 = 0, halo64 = 0;    // autotuned coupling kind per precision (0 nbr, 1/2 halo)
     int halo_hx = 0, halo_hy = 0, nwork = 0;
-    // separable coupling (coupling kind 3): p, q, kappa per z when every tap
-    // window factorises (see k_coupling_sep); host copies for the adjoint
+    // separable coupling (coupling kinds 3 to 5): p, q, kappa per z when every tap
+    // window factorises (see k_coupling_box); host copies for the adjoint
     bool sep_ok = false;
+    int box_h = 0;                     // window reach H of the box kernels (1, 2, 4 or 8)
+    struct SysBox { int x0, wx, y0, wy; bool wrapx, wrapy; };
+    std::vector<SysBox> sys_box;       // circular bounding box of each system's channels
+    struct Boxes {
+        DevBuf<msc::BoxWork> work;
+        int nwork = 0;
+        size_t smem = 0;           // the largest box's
+    } boxes[2][3];                     // [FP64, FP32][kind - 3], built when first used
     std::vector<double2> sep_p_h, sep_q_h, sep_k_h;   // [2hx+1][n], [2HY+1][n], [n]
     DevBuf<double2> sep64;                           // p | q | kappa
     DevBuf<float2> sep32;
@@ -281,6 +290,8 @@ struct msc_plan {
         gs_sys_lvl.release(); gs_lvl_start.release(); gs_lvl_rows.release();
         gs_low_ptr.release(); gs_low_tap.release(); gs_low_row.release();
         sep64.release(); sep32.release();
+        for (auto &row : boxes)
+            for (Boxes &b : row) b.work.release();
     }
 
     msc::Tiles tiles() const
@@ -546,83 +557,101 @@ void launch_halo_ys(msc_plan *p, const int *gate, const C2<R> *src, const C2<R> 
     }
 }
 
-size_t sep_smem(int hx, int hy, int zc, size_t elem)
+// The box kernel instance of (window reach, precision, kind) as a call of f(shape, kernel).
+template <typename R, int KIND, typename F>
+auto box_instance(int H, F f)
 {
-    const size_t hxw = kHaloBX + 2 * hx, hyw = 8 + 2 * hy;
-    return (hxw * hyw + (2 * hx + 1) + (2 * hy + 1) + 1) * zc * elem + hxw * hyw * sizeof(int);
+    using msc::BoxShape;
+    switch (H) {
+#define MSC_BOX_CASE(HH)                                                                          \
+    {                                                                                             \
+        using S = BoxShape<HH, R, KIND>;                                                          \
+        return f(S{}, &msc::k_coupling_box<HH, S::zc, R, S::seg, S::nt, S::minb, S::tm>);         \
+    }
+    case 1: MSC_BOX_CASE(1)
+    case 2: MSC_BOX_CASE(2)
+    case 4: MSC_BOX_CASE(4)
+    default: MSC_BOX_CASE(8)
+#undef MSC_BOX_CASE
+    }
 }
 
-template <int HY, int ZC, typename R>
-void launch_sep(msc_plan *p, const int *gate, const C2<R> *src, const C2<R> *in0, R sgn,
-                C2<R> *out, cudaStream_t st)
+template <typename R, typename F>
+auto box_instance(int H, int kind, F f)
 {
-    msc::CouplingTiles ct{p->work.p, p->pos_map.p, p->tap_window.p, p->nwork, p->nkx, p->nky,
-                          p->halo_hx, p->K};
-    const size_t np = (size_t)(2 * p->halo_hx + 1) * p->n, nq = (size_t)(2 * p->halo_hy + 1) * p->n;
-    const C2<R> *base = std::is_same<R, float>::value
-                            ? reinterpret_cast<const C2<R> *>(p->sep32.p)
-                            : reinterpret_cast<const C2<R> *>(p->sep64.p);
-    const msc::SepTaps sep{base, base + np, base + np + nq};
-    dim3 grid(p->nwork, (p->n + ZC - 1) / ZC);
-    const size_t sm = sep_smem(p->halo_hx, HY, ZC, sizeof(C2<R>));
-    if (p->halo_hx == HY)       // square window: the x reach at compile time
-        msc::k_coupling_sep<HY, kHaloBX, ZC, R, HY><<<grid, kHaloBX * ZC, sm, st>>>(
-            ct, gate, p->n, sep, src, in0, sgn, out);
-    else
-        msc::k_coupling_sep<HY, kHaloBX, ZC, R><<<grid, kHaloBX * ZC, sm, st>>>(
-            ct, gate, p->n, sep, src, in0, sgn, out);
+    if (kind == 3) return box_instance<R, 0>(H, f);
+    if (kind == 4) return box_instance<R, 1>(H, f);
+    return box_instance<R, 2>(H, f);
 }
 
-// The row-wise separable kernel: square windows (hx = hy), x reach as a
-// template parameter.
-bool sep_rows_ok(const msc_plan *p)
+// Work list of one kind: every system's box, cut along x past kBoxMaxX columns and
+// into as few strips of rows as its shared memory allows.
+template <typename R>
+msc_status ensure_boxes(msc_plan *p, int kind)
 {
-    return p->sep_ok && p->halo_hx == p->halo_hy &&
-           (p->halo_hx == 1 || p->halo_hx == 2 || p->halo_hx == 4 || p->halo_hx == 8);
-}
-
-template <int H, typename R>
-void launch_sep_rows_h(msc_plan *p, const int *gate, const C2<R> *src, const C2<R> *in0, R sgn,
-                       C2<R> *out, cudaStream_t st)
-{
-    constexpr int ZC = halo_zc<R>();
-    msc::CouplingTiles ct{p->work.p, p->pos_map.p, p->tap_window.p, p->nwork, p->nkx, p->nky,
-                          p->halo_hx, p->K};
-    const size_t np = (size_t)(2 * H + 1) * p->n, nq = (size_t)(2 * H + 1) * p->n;
-    const C2<R> *base = std::is_same<R, float>::value
-                            ? reinterpret_cast<const C2<R> *>(p->sep32.p)
-                            : reinterpret_cast<const C2<R> *>(p->sep64.p);
-    const msc::SepTaps sep{base, base + np, base + np + nq};
-    dim3 grid(p->nwork, (p->n + ZC - 1) / ZC);
-    msc::k_coupling_sep_rows<H, kHaloBX, ZC, R, H>
-        <<<grid, kHaloBX * ZC, sep_smem(H, H, ZC, sizeof(C2<R>)), st>>>(ct, gate, p->n, sep, src,
-                                                                        in0, sgn, out);
+    auto &bx = p->boxes[std::is_same<R, float>::value][kind - 3];
+    if (bx.nwork > 0) return MSC_OK;
+    const int H = p->box_h;
+    return box_instance<R>(H, kind, [&](auto shape, auto kernel) -> msc_status {
+        using S = decltype(shape);
+        std::vector<msc::BoxWork> wl;
+        size_t smem = 0;
+        for (int s = 0; s < p->B; ++s) {
+            const msc_plan::SysBox &b = p->sys_box[s];
+            const int kx = (b.wx + msc::kBoxMaxX - 1) / msc::kBoxMaxX;
+            const int nx = (b.wx + kx - 1) / kx;
+            int ky = 1, ny = b.wy;
+            bool strip = b.wrapy && b.wy < H;      // a wrap needs at least H rows to copy
+            auto fits = [&] {
+                const int wy = ny + (strip ? 2 * H : 0);
+                return S::smem(nx, wy) <= S::room;
+            };
+            while (!fits() && ny > 1) {
+                strip = true;
+                ++ky;
+                ny = (b.wy + ky - 1) / ky;
+            }
+            if (!fits()) return fail(MSC_ERR_DIMS, "coupling box does not fit in shared memory");
+            for (int x = 0; x < b.wx; x += nx)
+                for (int y = 0; y < b.wy; y += ny) {
+                    msc::BoxWork w;
+                    w.sys = s;
+                    w.wx = std::min(nx, b.wx - x);
+                    w.ny = std::min(ny, b.wy - y);
+                    w.strip = strip;
+                    w.wy = w.ny + (strip ? 2 * H : 0);
+                    w.xh = (((b.x0 + x - H) % p->nkx) + p->nkx) % p->nkx;
+                    w.y0 = (((b.y0 + y - (strip ? H : 0)) % p->nky) + p->nky) % p->nky;
+                    w.wrap = (b.wrapx || kx > 1 ? 1 : 0) | (b.wrapy && !strip ? 2 : 0);
+                    smem = std::max(smem, S::smem(w.wx, w.wy));
+                    wl.push_back(w);
+                }
+        }
+        MSC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::room));
+        MSC_CUDA(upload(bx.work, wl));
+        bx.nwork = (int)wl.size();
+        bx.smem = smem;
+        return MSC_OK;
+    });
 }
 
 template <typename R>
-void launch_sep_rows(msc_plan *p, const int *gate, const C2<R> *src, const C2<R> *in0, R sgn,
-                     C2<R> *out, cudaStream_t st)
+void launch_boxes(msc_plan *p, int kind, const int *gate, const C2<R> *src, const C2<R> *in0, R sgn,
+                  C2<R> *out, cudaStream_t st)
 {
-    switch (p->halo_hx) {
-    case 1: launch_sep_rows_h<1, R>(p, gate, src, in0, sgn, out, st); return;
-    case 2: launch_sep_rows_h<2, R>(p, gate, src, in0, sgn, out, st); return;
-    case 4: launch_sep_rows_h<4, R>(p, gate, src, in0, sgn, out, st); return;
-    default: launch_sep_rows_h<8, R>(p, gate, src, in0, sgn, out, st); return;
-    }
-}
-
-// ZC: z values per block (the halo kernel's, or half of it: half the shared
-// memory, twice the resident blocks to hide the halo loads)
-template <int ZC, typename R>
-void launch_sep_hy(msc_plan *p, const int *gate, const C2<R> *src, const C2<R> *in0, R sgn,
-                   C2<R> *out, cudaStream_t st)
-{
-    switch (p->halo_hy) {
-    case 1: launch_sep<1, ZC, R>(p, gate, src, in0, sgn, out, st); return;
-    case 2: launch_sep<2, ZC, R>(p, gate, src, in0, sgn, out, st); return;
-    case 4: launch_sep<4, ZC, R>(p, gate, src, in0, sgn, out, st); return;
-    default: launch_sep<8, ZC, R>(p, gate, src, in0, sgn, out, st); return;
-    }
+    const auto &bx = p->boxes[std::is_same<R, float>::value][kind - 3];
+    const size_t wn = (size_t)(2 * p->box_h + 1) * p->n;
+    const C2<R> *base = std::is_same<R, float>::value
+                            ? reinterpret_cast<const C2<R> *>(p->sep32.p)
+                            : reinterpret_cast<const C2<R> *>(p->sep64.p);
+    box_instance<R>(p->box_h, kind, [&](auto shape, auto kernel) {
+        using S = decltype(shape);
+        const int nzc = (p->n + S::zc - 1) / S::zc;
+        const msc::BoxArgs a{bx.work.p, p->pos_map.p, p->nkx, p->nky, nzc, base, base + wn,
+                             base + 2 * wn};
+        kernel<<<(unsigned)(bx.nwork * nzc), S::nt, bx.smem, st>>>(
+            a, gate, p->n, src, in0, sgn, out);
+    });
 }
 
 template <typename R>
@@ -630,23 +659,13 @@ void launch_coupling_t(msc_plan *p, const int *gate, const C2<R> *src, const C2<
                        C2<R> *out, cudaStream_t st)
 {
     // coupling kind per precision: 0 neighbour table, 1 halo (8 y/thread), 2 halo (4 y/thread),
-    // 3 separable (two 1-D passes; only when the tap windows factorise),
-    // 4 separable with half the z per block, 5 separable with the x pass
-    // along the halo rows (square windows; otherwise the column form)
+    // 3 to 5 separable over channel boxes (two 1-D passes; only when the tap windows
+    // factorise), with the most, half and a quarter of the z per block
     const int kind = p->use_halo ? (std::is_same<R, float>::value ? p->halo32 : p->halo64) : 0;
-    if (kind == 5 && p->sep_ok) {
-        if (sep_rows_ok(p)) launch_sep_rows<R>(p, gate, src, in0, sgn, out, st);
-        else launch_sep_hy<halo_zc<R>(), R>(p, gate, src, in0, sgn, out, st);
-        return;
-    }
     if (kind == 1) { launch_halo_ys<8, R>(p, gate, src, in0, sgn, out, st); return; }
     if (kind == 2) { launch_halo_ys<4, R>(p, gate, src, in0, sgn, out, st); return; }
-    if (kind == 3 && p->sep_ok) {
-        launch_sep_hy<halo_zc<R>(), R>(p, gate, src, in0, sgn, out, st);
-        return;
-    }
-    if (kind == 4 && p->sep_ok) {
-        launch_sep_hy<halo_zc<R>() / 2, R>(p, gate, src, in0, sgn, out, st);
+    if (kind >= 3 && p->sep_ok) {
+        launch_boxes<R>(p, kind, gate, src, in0, sgn, out, st);
         return;
     }
 
@@ -1040,37 +1059,6 @@ msc_status set_kernel_attributes(int n, int K)
     MSC_CUDA(cudaFuncSetAttribute(msc::k_coupling_halo<HY, kHaloBX, halo_zc<R>(), 4, R>,        \
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,                   \
                                   (int)std::min<size_t>(halo_smem(8, HY, halo_zc<R>(), sizeof(C2<R>)), 232448)));;
-#define MSC_SEP_ATTR(HY, R)                                                                      \
-    MSC_CUDA(cudaFuncSetAttribute(msc::k_coupling_sep<HY, kHaloBX, halo_zc<R>(), R>,              \
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,                   \
-                                  (int)std::min<size_t>(sep_smem(8, HY, halo_zc<R>(), sizeof(C2<R>)), 232448))); \
-    MSC_CUDA(cudaFuncSetAttribute(msc::k_coupling_sep<HY, kHaloBX, halo_zc<R>(), R, HY>,          \
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,                   \
-                                  (int)std::min<size_t>(sep_smem(HY, HY, halo_zc<R>(), sizeof(C2<R>)), 232448))); \
-    MSC_CUDA(cudaFuncSetAttribute(msc::k_coupling_sep<HY, kHaloBX, halo_zc<R>() / 2, R, HY>,      \
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,                   \
-                                  (int)std::min<size_t>(sep_smem(HY, HY, halo_zc<R>() / 2, sizeof(C2<R>)), 232448))); \
-    MSC_CUDA(cudaFuncSetAttribute(msc::k_coupling_sep<HY, kHaloBX, halo_zc<R>() / 2, R>,          \
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,                   \
-                                  (int)std::min<size_t>(sep_smem(8, HY, halo_zc<R>() / 2, sizeof(C2<R>)), 232448)));
-#define MSC_SEP_ROWS_ATTR(H, R)                                                                  \
-    MSC_CUDA(cudaFuncSetAttribute(msc::k_coupling_sep_rows<H, kHaloBX, halo_zc<R>(), R, H>,      \
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,                   \
-                                  (int)std::min<size_t>(sep_smem(H, H, halo_zc<R>(), sizeof(C2<R>)), 232448)));
-    MSC_SEP_ROWS_ATTR(1, float) MSC_SEP_ROWS_ATTR(2, float)
-    MSC_SEP_ROWS_ATTR(4, float) MSC_SEP_ROWS_ATTR(8, float)
-    MSC_SEP_ROWS_ATTR(1, double) MSC_SEP_ROWS_ATTR(2, double)
-    MSC_SEP_ROWS_ATTR(4, double) MSC_SEP_ROWS_ATTR(8, double)
-#undef MSC_SEP_ROWS_ATTR
-    MSC_SEP_ATTR(1, float)
-    MSC_SEP_ATTR(2, float)
-    MSC_SEP_ATTR(4, float)
-    MSC_SEP_ATTR(8, float)
-    MSC_SEP_ATTR(1, double)
-    MSC_SEP_ATTR(2, double)
-    MSC_SEP_ATTR(4, double)
-    MSC_SEP_ATTR(8, double)
-#undef MSC_SEP_ATTR
 #define MSC_HALO_MASK_ATTR(HY, R, M)                                                              \
     MSC_CUDA(cudaFuncSetAttribute(msc::k_coupling_halo<HY, kHaloBX, halo_zc<R>(), 4, R, M>,       \
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,                   \
@@ -1456,12 +1444,13 @@ msc_status autotune_measure(msc_plan *p)
     MSC_CUDA(cudaMemsetAsync(p->TMP.p, 0, vs * sizeof(double2), p->stream));
     const char *kind_name[6] = {"neighbour", "halo_y8", "halo_y4", "separable", "separable_z2",
                                 "separable_rows"};
-    const int nkinds = sep_rows_ok(p) ? 6 : p->sep_ok ? 5 : 3;
+    const int nkinds = p->sep_ok ? 6 : 3;
     if (p->use_halo) {
         float best = 0.f;
         int best_k = 0;
         for (int k = 0; k < nkinds; ++k) {
             p->halo64 = k;
+            if (k >= 3 && ensure_boxes<double>(p, k) != MSC_OK) continue;
             const float t = time_launch(p, [&](cudaStream_t st) {
                 launch_coupling_t<double>(p, nullptr, p->X.p, p->TMP.p, -1.0, p->TMP.p, st);
             });
@@ -1482,6 +1471,7 @@ msc_status autotune_measure(msc_plan *p)
             int best_k = 0;
             for (int k = 0; k < nkinds; ++k) {
                 p->halo32 = k;
+                if (k >= 3 && ensure_boxes<float>(p, k) != MSC_OK) continue;
                 const float t = time_launch(p, [&](cudaStream_t st) {
                     launch_coupling_t<float>(p, nullptr, a, c, 1.0f, b, st);
                 });
@@ -1629,19 +1619,18 @@ void separable_factors(msc_plan *p, const std::vector<int> &win)
 // at d is conj(V_{-d}): p_sdx -> conj(p_{-sdx}), q likewise, kappa -> conj).
 msc_status upload_separable(msc_plan *p)
 {
-    const int n = p->n, wx = 2 * p->halo_hx + 1, wy = 2 * p->halo_hy + 1;
-    std::vector<double2> all;
-    all.reserve((size_t)(wx + wy + 1) * n);
-    for (int a = 0; a < wx; ++a)
-        for (int z = 0; z < n; ++z) {
-            const double2 v = p->sep_p_h[(size_t)(p->adjoint ? wx - 1 - a : a) * n + z];
-            all.push_back(p->adjoint ? msc::cconj(v) : v);
-        }
-    for (int b = 0; b < wy; ++b)
-        for (int z = 0; z < n; ++z) {
-            const double2 v = p->sep_q_h[(size_t)(p->adjoint ? wy - 1 - b : b) * n + z];
-            all.push_back(p->adjoint ? msc::cconj(v) : v);
-        }
+    const int n = p->n, H = p->box_h, w = 2 * H + 1;
+    std::vector<double2> all((size_t)2 * w * n, double2{0.0, 0.0});   // zero past the windows' reach
+    all.reserve(all.size() + n);
+    auto fill = [&](const std::vector<double2> &src, int reach, size_t at) {
+        for (int d = -reach; d <= reach; ++d)
+            for (int z = 0; z < n; ++z) {
+                const double2 v = src[(size_t)(p->adjoint ? reach - d : reach + d) * n + z];
+                all[at + (size_t)(H + d) * n + z] = p->adjoint ? msc::cconj(v) : v;
+            }
+    };
+    fill(p->sep_p_h, p->halo_hx, 0);
+    fill(p->sep_q_h, p->halo_hy, (size_t)w * n);
     for (int z = 0; z < n; ++z) all.push_back(p->adjoint ? msc::cconj(p->sep_k_h[z]) : p->sep_k_h[z]);
     std::vector<float2> all32(all.size());
     for (size_t i = 0; i < all.size(); ++i) all32[i] = make_float2((float)all[i].x, (float)all[i].y);
@@ -1653,6 +1642,42 @@ msc_status upload_separable(msc_plan *p)
         MSC_CUDA(upload(p->sep32, all32));
     }
     return MSC_OK;
+}
+
+// Circular bounding box of each system's channels: the complement of the longest run
+// of free columns (rows).  With fewer than H free ones a box's two ends couple, and
+// the whole torus is taken, running around.
+void channel_boxes(msc_plan *p)
+{
+    const int H = p->box_h;
+    auto interval = [&](const std::vector<char> &occ, int &x0, int &w, bool &wrap) {
+        const int nk = (int)occ.size();
+        int best = 0, best_end = 0, run = 0;
+        for (int i = 0; i < 2 * nk; ++i) {
+            run = occ[i % nk] ? 0 : run + 1;
+            if (run > best && run < nk) {
+                best = run;
+                best_end = i % nk;
+            }
+        }
+        wrap = best < H;
+        x0 = wrap ? 0 : (best_end + 1) % nk;
+        w = wrap ? nk : nk - best;
+    };
+    p->sys_box.resize(p->B);
+    std::vector<char> ox(p->nkx), oy(p->nky);
+    for (int s = 0; s < p->B; ++s) {
+        const SystemHost &sh = p->sys[s];
+        std::fill(ox.begin(), ox.end(), 0);
+        std::fill(oy.begin(), oy.end(), 0);
+        for (int j = 0; j < sh.C; ++j) {
+            ox[sh.ix[j]] = 1;
+            oy[sh.iy[j]] = 1;
+        }
+        msc_plan::SysBox &b = p->sys_box[s];
+        interval(ox, b.x0, b.wx, b.wrapx);
+        interval(oy, b.y0, b.wy, b.wrapy);
+    }
 }
 
 msc_status finalize(msc_plan *p)
@@ -1790,6 +1815,9 @@ msc_status finalize(msc_plan *p)
             MSC_CUDA(upload(p->work, wl));
             separable_factors(p, win);
             if (p->sep_ok) {
+                p->box_h = 1;
+                while (p->box_h < std::max(hx, hyt)) p->box_h <<= 1;
+                channel_boxes(p);
                 msc_status sst = upload_separable(p);
                 if (sst != MSC_OK) return sst;
             }
@@ -1936,6 +1964,18 @@ msc_status finalize(msc_plan *p)
     {
         msc_status tst = autotune(p);
         if (tst != MSC_OK) return tst;
+    }
+    // the chosen forms' work lists (a choice from the cache or the environment); a
+    // box too wide for one form's shared memory takes the next, with fewer z per block
+    if (p->sep_ok && p->halo64 >= 3) {
+        msc_status bst = ensure_boxes<double>(p, p->halo64);
+        while (bst == MSC_ERR_DIMS && p->halo64 < 5) bst = ensure_boxes<double>(p, ++p->halo64);
+        if (bst != MSC_OK) return bst;
+    }
+    if (p->sep_ok && p->mixed && p->halo32 >= 3) {
+        msc_status bst = ensure_boxes<float>(p, p->halo32);
+        while (bst == MSC_ERR_DIMS && p->halo32 < 5) bst = ensure_boxes<float>(p, ++p->halo32);
+        if (bst != MSC_OK) return bst;
     }
     tm.mark("autotune");
     if (p->gs) {
