@@ -901,6 +901,45 @@ struct GmresState {
     int *counter;     // [1]  systems still unfinished (host reads it)
 };
 
+// What the host reads after a solve: one entry per system, and a last one with the
+// bounded waits' error words (status: tcgen05 inverse, unfinished: streamed passes).
+struct SolveReport {
+    int iters, projv, cycles, status, unfinished, pad;
+    double resid;
+};
+
+__global__ void k_solve_init(GmresState st, int nsys)
+{
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= nsys) return;
+    st.iters[s] = 0;
+    st.projv[s] = 0;
+    st.cycles[s] = 0;
+    st.status[s] = 0;
+    st.kcyc[s] = 0;
+    st.unfinished[s] = 1;
+}
+
+__global__ void k_solve_report(GmresState st, int nsys, const int *tc_error, const int *wait_error,
+                               SolveReport *out)
+{
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s > nsys) return;
+    SolveReport r{};
+    if (s == nsys) {
+        r.status = tc_error ? *tc_error : 0;
+        r.unfinished = *wait_error;
+    } else {
+        r.iters = st.iters[s];
+        r.projv = st.projv[s];
+        r.cycles = st.cycles[s];
+        r.status = st.status[s];
+        r.unfinished = st.unfinished[s];
+        r.resid = st.resid[s];
+    }
+    out[s] = r;
+}
+
 // Cycle start: norm of r = b - A x from the reduced partials (slot 0).
 __global__ void k_cycle_start(GmresState st, int nsys, int m, const double2 *__restrict__ nrm,
                               int nstride, double rtol, int max_iter, int max_cycles)

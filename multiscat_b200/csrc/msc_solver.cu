@@ -9,11 +9,11 @@
 // preconditioning and unrestarted MGS GMRES
 // (multiscat_gmres.f90:452-618); the converged psi is the same.
 //
-// Execution: one CUDA graph per restart cycle start (true residual + norm)
-// and one for the m Arnoldi steps + solution update.  Per-system activity
-// flags live on the device, so systems that converge early stop doing work
-// while the rest of the batch carries on.  The host reads one counter per
-// cycle.
+// Execution: one CUDA graph per restart cycle (the m Arnoldi steps, the solution
+// update, the next true residual and stop test); the first residual runs as plain
+// launches.  Per-system activity flags live on the device, so systems that converge
+// early stop doing work while the rest of the batch carries on.  The host reads one
+// counter per cycle.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -98,9 +98,15 @@ template <typename T>
 struct DevBuf {
     T *p = nullptr;
     size_t count = 0;
-    // Allocation and release are ordered on the legacy stream; alloc waits
-    // for the allocation, and the plan synchronises the device before it
-    // releases anything that work may still use.
+    DevBuf() = default;
+    DevBuf(const DevBuf &) = delete;
+    DevBuf &operator=(const DevBuf &) = delete;
+    ~DevBuf() { release(); }
+    // Allocation and release are ordered on the legacy stream, as the set-up's
+    // copies and kernels are; whoever uses a new buffer on another stream waits
+    // for the legacy one first (finalize does so once for the whole plan).  The
+    // plan synchronises the device before it releases anything that work may
+    // still use.
     cudaError_t alloc(size_t c)
     {
         release();
@@ -125,7 +131,7 @@ struct DevBuf {
             e = cudaMemsetAsync(p, 0xff, c * sizeof(T), 0);
             if (e != cudaSuccess) return e;
         }
-        return cudaStreamSynchronize(0);
+        return cudaSuccess;
     }
     void release()
     {
@@ -134,6 +140,80 @@ struct DevBuf {
         count = 0;
     }
 };
+
+// A plan's stream and pinned host block.  cudaMallocHost, cudaFreeHost and the
+// stream calls cost 2 to 5 ms per plan (the whole one-beam solve takes less), so a
+// destroyed plan's pair goes to a list per device, from which the next plan takes
+// the smallest that is large enough.  At most kIdleKits idle pairs of at most
+// kIdleKitBytes each are kept; msc_release_cached_memory frees those of its device.
+// A plan returns its pair after synchronising, so it comes back idle.
+struct PlanKit {
+    int dev = -1;
+    cudaStream_t stream = nullptr;
+    unsigned char *pinned = nullptr;
+    size_t bytes = 0;
+};
+constexpr size_t kIdleKits = 16;
+constexpr size_t kIdleKitBytes = 1u << 20;
+std::mutex g_kit_mutex;
+std::vector<PlanKit> &idle_kits()
+{
+    static auto *kits = new std::vector<PlanKit>();     // never destroyed: outlives every plan
+    return *kits;
+}
+
+void kit_free(PlanKit &k)
+{
+    if (k.pinned) cudaFreeHost(k.pinned);
+    if (k.stream) cudaStreamDestroy(k.stream);
+    k = PlanKit{};
+}
+
+cudaError_t kit_acquire(size_t bytes, PlanKit *out)
+{
+    int dev = -1;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    {
+        std::lock_guard<std::mutex> lock(g_kit_mutex);
+        auto &kits = idle_kits();
+        auto best = kits.end();
+        for (auto it = kits.begin(); it != kits.end(); ++it)
+            if (it->dev == dev && it->bytes >= bytes && (best == kits.end() || it->bytes < best->bytes))
+                best = it;
+        if (best != kits.end()) {
+            *out = *best;
+            kits.erase(best);
+            return cudaSuccess;
+        }
+    }
+    PlanKit k;
+    k.dev = dev;
+    k.bytes = 4096;
+    while (k.bytes < bytes) k.bytes *= 2;
+    e = cudaStreamCreateWithFlags(&k.stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void **>(&k.pinned), k.bytes);
+    if (e != cudaSuccess) {
+        kit_free(k);
+        return e;
+    }
+    *out = k;
+    return cudaSuccess;
+}
+
+void kit_return(PlanKit &k)
+{
+    if (!k.stream) return;
+    if (k.bytes <= kIdleKitBytes) {
+        std::lock_guard<std::mutex> lock(g_kit_mutex);
+        if (idle_kits().size() < kIdleKits) {
+            idle_kits().push_back(k);
+            k = PlanKit{};
+            return;
+        }
+    }
+    kit_free(k);
+}
 
 struct SystemHost {
     int C = 0;
@@ -214,7 +294,10 @@ struct msc_plan {
     DevBuf<__nv_bfloat16> e_img;
     DevBuf<int> tc_error;
     DevBuf<int> active, kcyc, iters, projv, cycles, unfinished, status, counter;
-    int *counter_host = nullptr;   // pinned
+    int *counter_host = nullptr;   // pinned (in kit)
+    PlanKit kit;
+    DevBuf<msc::SolveReport> report;              // [B + 1] results of a solve, error words last
+    msc::SolveReport *report_host = nullptr;      // pinned (in kit)
     // Arnoldi blocks: runs of rows of one system ("chunks", first projection)
     // and row tiles split `split` ways (update + second projection)
     int nchunks = 0;
@@ -245,7 +328,7 @@ struct msc_plan {
     DevBuf<int2> taps_d;                      // [K] tap offsets (dx, dy)
     DevBuf<int> sys_counter;       // per-system arrival counters of the fused Arnoldi kernels
     cudaStream_t stream = nullptr;
-    cudaGraphExec_t g_start = nullptr, g_start0 = nullptr, g_iter = nullptr;
+    cudaGraphExec_t g_cycle = nullptr;   // the m Arnoldi steps of a cycle and the next cycle's start
     int pstride = 0;
     // measurement
     bool timing = false;
@@ -253,45 +336,17 @@ struct msc_plan {
     std::vector<cudaEvent_t> tev;        // [kKinds][m + 1 slots][start, stop]
     double t_ms[kKinds] = {};
     int64_t t_launches[kKinds] = {};
-    int *kcyc_host = nullptr;            // pinned [B]
+    int *kcyc_host = nullptr;            // pinned [B] (in kit)
     int64_t launches_last = 0;
     int cycles_last = 0;
     int fallbacks_last = 0;              // systems re-solved in FP64 by the last msc_solve
-    int64_t launches_start = 0, launches_start0 = 0, launches_iter = 0;   // kernel nodes per graph
+    int64_t launches_cycle = 0;          // kernel nodes of the cycle graph
 
     ~msc_plan()
     {
-        if (g_start) cudaGraphExecDestroy(g_start);
-        if (g_start0) cudaGraphExecDestroy(g_start0);
-        if (g_iter) cudaGraphExecDestroy(g_iter);
-        if (counter_host) cudaFreeHost(counter_host);
-        if (kcyc_host) cudaFreeHost(kcyc_host);
+        if (g_cycle) cudaGraphExecDestroy(g_cycle);
         for (cudaEvent_t e : tev) cudaEventDestroy(e);
-        if (stream) cudaStreamDestroy(stream);
-        E.release(); Tm.release(); lam.release(); en.release(); v00.release();
-        row_pkd.release(); row_fn.release(); Vt.release(); row_c.release(); row_b.release();
-        row_cf.release(); img_et.release(); img_e.release(); img_t.release();
-        row_rhs.release(); sys_aspec.release(); row_pos.release(); pos_map.release();
-        sys_row0.release(); nbr.release(); tile_row0.release();
-        tile_nrow.release(); tile_sys.release(); sys_tile0.release(); sys_spec_row.release();
-        chunk_row0.release(); chunk_nrow.release(); chunk_sys.release(); sys_chunk0.release();
-        row_sys.release(); X.release(); W.release(); U.release(); TMP.release(); Q.release();
-        partial.release(); H.release(); cs.release(); sn.release(); g.release(); h1.release();
-        h2.release(); y.release(); scale.release(); bnorm.release(); resid.release();
-        est.release(); active.release(); kcyc.release(); iters.release(); projv.release();
-        cycles.release();
-        unfinished.release(); status.release(); counter.release(); beta0.release();
-        sys_counter.release(); work.release(); tap_window.release(); taps_d.release();
-        E32.release(); ET32.release(); lam32.release(); en32.release(); row_pkd32.release();
-        row_fn32.release(); Vt32.release(); row_c32.release(); Q32.release(); W32.release();
-        T32.release(); T64.release(); X0.release();
-        U32.release(); R64.release(); e_img.release(); e_img_kz.release(); e_img_zk.release(); tc_error.release(); wait_error.release();
-        Hraw.release(); dsum.release(); dcoef.release(); gsave.release();
-        gs_sys_lvl.release(); gs_lvl_start.release(); gs_lvl_rows.release();
-        gs_low_ptr.release(); gs_low_tap.release(); gs_low_row.release();
-        sep64.release(); sep32.release();
-        for (auto &row : boxes)
-            for (Boxes &b : row) b.work.release();
+        kit_return(kit);
     }
 
     msc::Tiles tiles() const
@@ -329,7 +384,8 @@ cudaError_t upload(DevBuf<T> &buf, const std::vector<T> &h)
     cudaError_t e = buf.alloc(h.size());
     if (e != cudaSuccess) return e;
     if (h.empty()) return cudaSuccess;
-    return cudaMemcpy(buf.p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice);
+    // (pageable source: it has been read when the call returns)
+    return cudaMemcpyAsync(buf.p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, 0);
 }
 
 // Overwrite an allocated buffer in place (device pointers captured in the
@@ -385,28 +441,30 @@ constexpr int kTcChannelMajor = 3;
 // ... and of the form with E streamed from L2 (k_block_inverse_tcs)
 constexpr int kTcStream = 4;
 
-// One instance of the streamed kernel: its launch, or (attr) its shared-memory limit.
+// One instance of the streamed kernel: its launch, or (limit > 0) its shared-memory
+// limit.  (Limits are set to what the device allows, not to one plan's need, so that
+// no plan lowers another's.)
 template <int N, int S>
-cudaError_t tcs_instance(const msc::tc::TcStreamParams &sp, int grid, cudaStream_t st, bool attr)
+cudaError_t tcs_instance(const msc::tc::TcStreamParams &sp, int grid, cudaStream_t st, int limit)
 {
-    const size_t bytes = msc::tc::stream_smem(sp.t.kp, N, S);
-    if (attr)
+    if (limit > 0)
         return cudaFuncSetAttribute(msc::tc::k_block_inverse_tcs<N, S>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    msc::tc::k_block_inverse_tcs<N, S><<<grid, msc::tc::kThreads, bytes, st>>>(sp);
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+    msc::tc::k_block_inverse_tcs<N, S>
+        <<<grid, msc::tc::kThreads, msc::tc::stream_smem(sp.t.kp, N, S), st>>>(sp);
     return cudaGetLastError();
 }
 
-cudaError_t tcs_dispatch(int N, int S, const msc::tc::TcStreamParams &sp, int grid, cudaStream_t st, bool attr)
+cudaError_t tcs_dispatch(int N, int S, const msc::tc::TcStreamParams &sp, int grid, cudaStream_t st, int limit)
 {
     if (N == 128) {
-        if (S == 4) return tcs_instance<128, 4>(sp, grid, st, attr);
-        if (S == 3) return tcs_instance<128, 3>(sp, grid, st, attr);
-        return tcs_instance<128, 2>(sp, grid, st, attr);
+        if (S == 4) return tcs_instance<128, 4>(sp, grid, st, limit);
+        if (S == 3) return tcs_instance<128, 3>(sp, grid, st, limit);
+        return tcs_instance<128, 2>(sp, grid, st, limit);
     }
-    if (S == 4) return tcs_instance<64, 4>(sp, grid, st, attr);
-    if (S == 3) return tcs_instance<64, 3>(sp, grid, st, attr);
-    return tcs_instance<64, 2>(sp, grid, st, attr);
+    if (S == 4) return tcs_instance<64, 4>(sp, grid, st, limit);
+    if (S == 3) return tcs_instance<64, 3>(sp, grid, st, limit);
+    return tcs_instance<64, 2>(sp, grid, st, limit);
 }
 
 void launch_block_inverse_tc(msc_plan *p, const int *gate, const float2 *x, float2 *out,
@@ -433,7 +491,7 @@ void launch_block_inverse_tc(msc_plan *p, const int *gate, const float2 *x, floa
     constexpr int T = msc::tc::kThreads;
     if (p->tc_groups == kTcStream) {
         const msc::tc::TcStreamParams sp{prm, p->e_img_zk.p, p->e_img_kz.p};
-        (void)tcs_dispatch(p->tc_n, p->tcs_stages[p->tc_n == 128], sp, p->tc_grid, st, false);
+        (void)tcs_dispatch(p->tc_n, p->tcs_stages[p->tc_n == 128], sp, p->tc_grid, st, 0);
         return;
     }
     if (p->tc_groups == kTcChannelMajor) {
@@ -821,11 +879,8 @@ void record_cycle_start_t(msc_plan *p, bool x_zero, cudaStream_t st)
     cudaMemcpyAsync(p->counter_host, p->counter.p, sizeof(int), cudaMemcpyDeviceToHost, st);
 }
 
-void record_cycle_start(msc_plan *p, cudaStream_t st) { record_cycle_start_t(p, false, st); }
-
-// First cycle of a solve from x = 0 (no warm start): r = b without the
-// residual's T GEMM and FP64 coupling.
-void record_cycle_start_zero(msc_plan *p, cudaStream_t st) { record_cycle_start_t(p, true, st); }
+// Kernels of a cycle start.
+int64_t cycle_start_launches(bool x_zero) { return x_zero ? 5 : 6; }
 
 // m Arnoldi steps (CGS2) in precision R and the solution update x += M (Q y).
 // out = M x with the von Neumann preconditioner of order k,
@@ -981,6 +1036,14 @@ void record_cycle_iterations(msc_plan *p, cudaStream_t st)
         record_iterations_t<double>(p, p->Q.p, p->W.p, p->U.p, st);
 }
 
+// One graph per restart cycle: its Arnoldi steps, the solution update and the next
+// cycle's start (true residual, stop test), so that the host waits once a cycle.
+void record_cycle(msc_plan *p, cudaStream_t st)
+{
+    record_cycle_iterations(p, st);
+    record_cycle_start_t(p, false, st);
+}
+
 // Kernel nodes in a captured graph (launch accounting).
 int64_t count_kernel_nodes(cudaGraph_t g)
 {
@@ -1041,8 +1104,16 @@ msc_status capture(msc_plan *p, void (*rec)(msc_plan *, cudaStream_t), cudaGraph
     return MSC_OK;
 }
 
-msc_status set_kernel_attributes(int n, int K)
+// Shared-memory limits of the kernels on the current device, set once per process.
+msc_status set_kernel_attributes()
 {
+    static std::mutex mutex;
+    static bool done[kPoolMaxDevices] = {};
+    int dev = -1;
+    MSC_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= kPoolMaxDevices) return fail(MSC_ERR_CUDA, "device index out of range");
+    std::lock_guard<std::mutex> lock(mutex);
+    if (done[dev]) return MSC_OK;
     MSC_CUDA(msc::dm::set_attributes());
     MSC_CUDA(cudaFuncSetAttribute(msc::k_block_inverse<8, float>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1085,8 +1156,17 @@ msc_status set_kernel_attributes(int n, int K)
                                   (int)smem_residual(msc::kMaxNz)));
     MSC_CUDA(cudaFuncSetAttribute(msc::k_coupling<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)smem_coupling(msc::kMaxTaps)));
-    (void)n;
-    (void)K;
+    // the register-streamed reduction's last block stages its scalar work in
+    // dynamic shared memory (up to the largest restart)
+    MSC_CUDA(cudaFuncSetAttribute(msc::k_dcgs_reduce<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)dcgs_scratch_bytes(msc::kMaxRestart)));
+    MSC_CUDA(cudaFuncSetAttribute(msc::k_dcgs_reduce<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)dcgs_scratch_bytes(msc::kMaxRestart)));
+    MSC_CUDA(cudaFuncSetAttribute(msc::k_dcgs_reduce_bulk, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)msc::dcgs_bulk_smem()));
+    MSC_CUDA(cudaFuncSetAttribute(msc::k_dcgs_update_bulk, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)msc::dcgs_bulk_smem()));
+    done[dev] = true;
     return MSC_OK;
 }
 
@@ -1180,7 +1260,7 @@ size_t tc_request_bytes(int n, int N, int G)
 // form, 32 or 64 channels per tile, as many ring stages (up to 4) as fit.
 msc_status setup_tc_stream(msc_plan *p, int sms, size_t optin)
 {
-    const int n = p->n, kp = (n + 15) / 16 * 16, kb = kp / 8, mt = (n + 127) / 128;
+    const int n = p->n, kp = (n + 15) / 16 * 16, mt = (n + 127) / 128;
     cudaFuncAttributes fa{};
     MSC_CUDA(cudaFuncGetAttributes(&fa, msc::tc::k_block_inverse_tcs<128, 4>));
     msc::tc::TcStreamParams sp{};
@@ -1193,7 +1273,7 @@ msc_status setup_tc_stream(msc_plan *p, int sms, size_t optin)
         for (int S = 4; S >= 2 && !p->tcs_stages[w]; --S)
             if (msc::tc::stream_smem(kp, N, S) + fa.sharedSizeBytes <= optin) p->tcs_stages[w] = S;
         if (!p->tcs_stages[w]) continue;
-        MSC_CUDA(tcs_dispatch(N, p->tcs_stages[w], sp, 0, nullptr, true));
+        MSC_CUDA(tcs_dispatch(N, p->tcs_stages[w], sp, 0, nullptr, (int)optin - (int)fa.sharedSizeBytes));
         p->tc_n = N;       // the widest that fits; the autotuner times both
     }
     if (p->tc_n == 0) return MSC_OK;
@@ -1201,27 +1281,12 @@ msc_status setup_tc_stream(msc_plan *p, int sms, size_t optin)
     p->tc_tile_rows = p->tc_n / 2;
     p->tc_ntiles = (p->R + p->tc_tile_rows - 1) / p->tc_tile_rows;
     p->tc_grid = std::min(p->tc_ntiles, sms);
-    // operand images, one contiguous piece [hi, lo][2 K blocks][M blocks][8 z][8 k]
-    // per 16 of K: K = z for E^T x, K = k for E y
-    std::vector<__nv_bfloat16> zk((size_t)2 * kp * kp, __float2bfloat16(0.f)), kz(zk);
-    const size_t part = (size_t)16 * kp;
-    for (int z = 0; z < n; ++z)
-        for (int k = 0; k < n; ++k) {
-            const double v = p->E_host[(size_t)z * n + k];
-            const __nv_bfloat16 hi = __float2bfloat16_rn((float)v);
-            const __nv_bfloat16 lo = __float2bfloat16_rn((float)(v - (double)__bfloat162float(hi)));
-            const size_t in = (size_t)(z % 8) * 8 + k % 8;
-            const size_t a = (size_t)(z / 16) * 2 * part + ((size_t)(z / 8 % 2) * kb + k / 8) * 64 + in;
-            const size_t b = (size_t)(k / 16) * 2 * part + ((size_t)(k / 8 % 2) * kb + z / 8) * 64 + in;
-            zk[a] = hi;
-            zk[a + part] = lo;
-            kz[b] = hi;
-            kz[b + part] = lo;
-        }
-    MSC_CUDA(upload(p->e_img_zk, zk));
-    MSC_CUDA(upload(p->e_img_kz, kz));
+    MSC_CUDA(p->e_img_zk.alloc((size_t)2 * kp * kp));
+    MSC_CUDA(p->e_img_kz.alloc((size_t)2 * kp * kp));
+    msc::tc::k_stream_images<<<(kp * kp + 255) / 256, 256>>>(n, kp, p->E.p, p->e_img_zk.p, p->e_img_kz.p);
+    MSC_CUDA(cudaGetLastError());
     MSC_CUDA(p->tc_error.alloc(1));
-    MSC_CUDA(cudaMemset(p->tc_error.p, 0, sizeof(int)));
+    MSC_CUDA(cudaMemsetAsync(p->tc_error.p, 0, sizeof(int), 0));
     p->use_tc = true;
     return MSC_OK;
 }
@@ -1259,7 +1324,7 @@ msc_status setup_tensor_core(msc_plan *p)
     p->tc_smem = tc_request_bytes(n, chosen, 1);
     if (p->tc_smem + tc_static_for(chosen) > (size_t)optin) return MSC_OK;
     for (int N = 16; N <= chosen; N *= 2) {
-        cudaError_t e = tc_set_smem_for(N, 1, p->tc_smem);
+        cudaError_t e = tc_set_smem_for(N, 1, (size_t)optin - tc_static_for(N));
         if (e != cudaSuccess) return fail(MSC_ERR_CUDA, std::string("tc smem attribute: ") + cudaGetErrorString(e));
     }
     // two-group variants: widths whose two TMEM regions and two B buffers fit
@@ -1272,7 +1337,7 @@ msc_status setup_tensor_core(msc_plan *p)
     if (p->tc2_max > 0) {
         p->tc2_smem = tc_request_bytes(n, p->tc2_max, 2);
         for (int N = 16; N <= p->tc2_max; N *= 2) {
-            cudaError_t e = tc_set_smem_for(N, 2, p->tc2_smem);
+            cudaError_t e = tc_set_smem_for(N, 2, (size_t)optin - tc_static_for(N, 2));
             if (e != cudaSuccess) return fail(MSC_ERR_CUDA, std::string("tc smem attribute: ") + cudaGetErrorString(e));
         }
     }
@@ -1287,25 +1352,16 @@ msc_status setup_tensor_core(msc_plan *p)
         if (p->tcc_ok) {
             cudaError_t e = cudaFuncSetAttribute(msc::tc::k_block_inverse_tcc,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)p->tcc_smem);
+                                                 optin - (int)fa.sharedSizeBytes);
             if (e != cudaSuccess) return fail(MSC_ERR_CUDA, std::string("tcc smem attribute: ") + cudaGetErrorString(e));
         }
     }
-    // E image: [hi|lo][z/8][k/8][z%8][k%8], zero padded to kp x kp
-    const int kp = (n + 15) / 16 * 16, kb = kp / 8;
-    std::vector<__nv_bfloat16> img((size_t)2 * kp * kp, __float2bfloat16(0.f));
-    for (int z = 0; z < n; ++z)
-        for (int k = 0; k < n; ++k) {
-            const double v = p->E_host[(size_t)z * n + k];
-            const __nv_bfloat16 hi = __float2bfloat16_rn((float)v);
-            const __nv_bfloat16 lo = __float2bfloat16_rn((float)(v - (double)__bfloat162float(hi)));
-            const size_t off = ((size_t)(z / 8) * kb + k / 8) * 64 + (z % 8) * 8 + (k % 8);
-            img[off] = hi;
-            img[(size_t)kp * kp + off] = lo;
-        }
-    MSC_CUDA(upload(p->e_img, img));
+    const int kp = (n + 15) / 16 * 16;
+    MSC_CUDA(p->e_img.alloc((size_t)2 * kp * kp));
+    msc::tc::k_resident_image<<<(kp * kp + 255) / 256, 256>>>(n, kp, p->E.p, p->e_img.p);
+    MSC_CUDA(cudaGetLastError());
     MSC_CUDA(p->tc_error.alloc(1));
-    MSC_CUDA(cudaMemset(p->tc_error.p, 0, sizeof(int)));
+    MSC_CUDA(cudaMemsetAsync(p->tc_error.p, 0, sizeof(int), 0));
     p->use_tc = true;
     return MSC_OK;
 }
@@ -1756,7 +1812,7 @@ msc_status finalize(msc_plan *p)
     }
     MSC_CUDA(p->row_fn.alloc(p->R));
     MSC_CUDA(p->nbr.alloc((size_t)p->R * std::max(p->K, 1)));
-    if (p->K == 0) MSC_CUDA(cudaMemset(p->nbr.p, 0xff, p->nbr.count * sizeof(int)));
+    if (p->K == 0) MSC_CUDA(cudaMemsetAsync(p->nbr.p, 0xff, p->nbr.count * sizeof(int), 0));
     if (p->mixed) MSC_CUDA(p->row_fn32.alloc(p->R));
     msc::k_row_tables<<<std::min((p->R + 255) / 256, 4096), 256>>>(
         p->R, n, p->K, p->nkx, p->nky, p->row_pos.p, p->row_sys.p, p->pos_map.p, p->taps_d.p,
@@ -1767,7 +1823,6 @@ msc_status finalize(msc_plan *p)
     msc::k_row_cfac<<<std::min((p->R + 255) / 256, 4096), 256>>>(p->R, p->row_c.p, p->row_fn.p,
                                                                  p->row_cf.p);
     MSC_CUDA(cudaGetLastError());
-    MSC_CUDA(cudaDeviceSynchronize());
     tm.mark("row tables (device)");
     {
         // Halo-tiled coupling: signed tap reach, tap window, position->row
@@ -1896,21 +1951,7 @@ msc_status finalize(msc_plan *p)
         if (bulk_ok && rmode && std::strcmp(rmode, "registers") == 0) p->bulk_arnoldi = 0;
         if (bulk_ok && rmode && std::strcmp(rmode, "reduce") == 0) p->bulk_arnoldi = 1;
         MSC_CUDA(p->wait_error.alloc(1));
-        MSC_CUDA(cudaMemset(p->wait_error.p, 0, sizeof(int)));
-        // the register-streamed reduction's last block stages its scalar work
-        // in dynamic shared memory (up to the largest restart)
-        MSC_CUDA(cudaFuncSetAttribute(msc::k_dcgs_reduce<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)dcgs_scratch_bytes(msc::kMaxRestart)));
-        MSC_CUDA(cudaFuncSetAttribute(msc::k_dcgs_reduce<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)dcgs_scratch_bytes(msc::kMaxRestart)));
-        if (p->bulk_arnoldi > 0)
-            MSC_CUDA(cudaFuncSetAttribute(msc::k_dcgs_reduce_bulk,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)msc::dcgs_bulk_smem()));
-        if (p->bulk_arnoldi > 1)
-            MSC_CUDA(cudaFuncSetAttribute(msc::k_dcgs_update_bulk,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)msc::dcgs_bulk_smem()));
+        MSC_CUDA(cudaMemsetAsync(p->wait_error.p, 0, sizeof(int), 0));
         MSC_CUDA(upload(p->chunk_row0, c0));
         MSC_CUDA(upload(p->chunk_nrow, cn));
         MSC_CUDA(upload(p->chunk_sys, cs));
@@ -1925,7 +1966,7 @@ msc_status finalize(msc_plan *p)
     }
     MSC_CUDA(p->partial.alloc((size_t)std::max(p->ntiles * p->split, p->nchunks) * p->pstride));
     MSC_CUDA(p->sys_counter.alloc(p->B));
-    MSC_CUDA(cudaMemset(p->sys_counter.p, 0, p->B * sizeof(int)));
+    MSC_CUDA(cudaMemsetAsync(p->sys_counter.p, 0, p->B * sizeof(int), 0));
     MSC_CUDA(p->H.alloc((size_t)p->B * (m + 1) * m));
     MSC_CUDA(p->cs.alloc((size_t)p->B * m));
     MSC_CUDA(p->sn.alloc((size_t)p->B * m));
@@ -1937,8 +1978,8 @@ msc_status finalize(msc_plan *p)
     MSC_CUDA(p->dsum.alloc((size_t)p->B * 2 * (m + 1)));
     MSC_CUDA(p->dcoef.alloc((size_t)p->B * (2 * m + 4)));
     MSC_CUDA(p->gsave.alloc(p->B));
-    MSC_CUDA(cudaMemset(p->Hraw.p, 0, p->Hraw.count * sizeof(double2)));
-    MSC_CUDA(cudaMemset(p->dcoef.p, 0, p->dcoef.count * sizeof(double2)));
+    MSC_CUDA(cudaMemsetAsync(p->Hraw.p, 0, p->Hraw.count * sizeof(double2), 0));
+    MSC_CUDA(cudaMemsetAsync(p->dcoef.p, 0, p->dcoef.count * sizeof(double2), 0));
     MSC_CUDA(p->scale.alloc(p->B));
     MSC_CUDA(p->resid.alloc(p->B));
     MSC_CUDA(p->beta0.alloc(p->B));
@@ -1951,9 +1992,9 @@ msc_status finalize(msc_plan *p)
     MSC_CUDA(p->unfinished.alloc(p->B));
     MSC_CUDA(p->status.alloc(p->B));
     MSC_CUDA(p->counter.alloc(1));
-    MSC_CUDA(cudaMemset(p->H.p, 0, p->H.count * sizeof(double2)));
-    MSC_CUDA(cudaMemset(p->h1.p, 0, p->h1.count * sizeof(double2)));
-    MSC_CUDA(cudaMemset(p->y.p, 0, p->y.count * sizeof(double2)));
+    MSC_CUDA(cudaMemsetAsync(p->H.p, 0, p->H.count * sizeof(double2), 0));
+    MSC_CUDA(cudaMemsetAsync(p->h1.p, 0, p->h1.count * sizeof(double2), 0));
+    MSC_CUDA(cudaMemsetAsync(p->y.p, 0, p->y.count * sizeof(double2), 0));
 
     tm.mark("solver allocations");
     {
@@ -1961,6 +2002,7 @@ msc_status finalize(msc_plan *p)
         if (tst != MSC_OK) return tst;
     }
     tm.mark("tensor-core setup");
+    MSC_CUDA(cudaStreamSynchronize(0));      // the autotuner launches on the plan's stream
     {
         msc_status tst = autotune(p);
         if (tst != MSC_OK) return tst;
@@ -1983,15 +2025,10 @@ msc_status finalize(msc_plan *p)
         if (gst != MSC_OK) return gst;
         tm.mark("Gauss-Seidel levels");
     }
-    MSC_CUDA(cudaMallocHost(&p->kcyc_host, p->B * sizeof(int)));
     for (int s = 0; s < p->B; ++s) p->kcyc_host[s] = 0;
-    p->tev.resize((size_t)msc_plan::kKinds * (m + 1) * 2);
-    for (cudaEvent_t &e : p->tev) MSC_CUDA(cudaEventCreate(&e));
-    msc_status st = capture(p, record_cycle_start, &p->g_start, &p->launches_start);
-    if (st != MSC_OK) return st;
-    st = capture(p, record_cycle_start_zero, &p->g_start0, &p->launches_start0);
-    if (st != MSC_OK) return st;
-    st = capture(p, record_cycle_iterations, &p->g_iter, &p->launches_iter);
+    MSC_CUDA(p->report.alloc(p->B + 1));
+    MSC_CUDA(cudaStreamSynchronize(0));      // everything above is in place for the plan's stream
+    msc_status st = capture(p, record_cycle, &p->g_cycle, &p->launches_cycle);
     if (st != MSC_OK) return st;
     tm.mark("graph capture");
     p->finalized = true;
@@ -2065,9 +2102,9 @@ msc_status ensure_gs_levels(msc_plan *p)
     p->gs_e64_smem = gs_smem<double>(p->n, true) <= room;
     p->gs_e32_smem = p->E32.p && gs_smem<float>(p->n, true) <= room;
     MSC_CUDA(cudaFuncSetAttribute(msc::k_gs_sweep<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)gs_smem<double>(p->n, p->gs_e64_smem)));
+                                  (int)room));
     MSC_CUDA(cudaFuncSetAttribute(msc::k_gs_sweep<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)gs_smem<float>(p->n, p->gs_e32_smem)));
+                                  (int)room));
     MSC_CUDA(cudaFuncSetAttribute(msc::k_coupling_masked<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)smem_coupling(msc::kMaxTaps)));
     MSC_CUDA(cudaFuncSetAttribute(msc::k_coupling_masked<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2091,8 +2128,8 @@ msc_status device_symmetric_eigh(int n, const double *H, double *w, double *E)
     MSC_CUDA(d.alloc(n));
     MSC_CUDA(e.alloc(n));
     MSC_CUDA(applied.alloc(n));
-    MSC_CUDA(cudaMemset(R.p, 0, (size_t)n * n * sizeof(double)));
-    MSC_CUDA(cudaMemset(e.p, 0, (size_t)n * sizeof(double)));
+    MSC_CUDA(cudaMemsetAsync(R.p, 0, (size_t)n * n * sizeof(double), 0));
+    MSC_CUDA(cudaMemsetAsync(e.p, 0, (size_t)n * sizeof(double), 0));
     const size_t tri_smem = n <= eg::kTriSmemMaxN ? (size_t)n * n * sizeof(double) : 0;
     MSC_CUDA(cudaFuncSetAttribute(eg::k_tridiagonalize, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)((size_t)eg::kTriSmemMaxN * eg::kTriSmemMaxN * sizeof(double))));
@@ -2120,12 +2157,12 @@ msc_status device_symmetric_eigh(int n, const double *H, double *w, double *E)
     if ((size_t)n * 32 * sizeof(double) <= 200 * 1024) {
         const size_t sm = (size_t)n * 32 * sizeof(double);
         MSC_CUDA(cudaFuncSetAttribute(eg::k_apply_rotations<32>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         eg::k_apply_rotations<32><<<(n + 31) / 32, 32, sm>>>(n, nrot, rk.p, rc.p, rs.p, Zt.p);
     } else {
         const size_t sm = (size_t)n * 16 * sizeof(double);
         MSC_CUDA(cudaFuncSetAttribute(eg::k_apply_rotations<16>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         eg::k_apply_rotations<16><<<(n + 15) / 16, 16, sm>>>(n, nrot, rk.p, rc.p, rs.p, Zt.p);
     }
     MSC_CUDA(cudaGetLastError());
@@ -2142,12 +2179,12 @@ msc_status device_symmetric_eigh(int n, const double *H, double *w, double *E)
     if ((size_t)n * 32 * sizeof(double) <= 200 * 1024) {
         const size_t sm = (size_t)n * 32 * sizeof(double);
         MSC_CUDA(cudaFuncSetAttribute(eg::k_back_transform<32>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         eg::k_back_transform<32><<<(n + 31) / 32, 256, sm>>>(n, R.p, applied.p, Zt.p, dest.p, Ed.p);
     } else {
         const size_t sm = (size_t)n * 16 * sizeof(double);
         MSC_CUDA(cudaFuncSetAttribute(eg::k_back_transform<16>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         eg::k_back_transform<16><<<(n + 15) / 16, 256, sm>>>(n, R.p, applied.p, Zt.p, dest.p, Ed.p);
     }
     MSC_CUDA(cudaGetLastError());
@@ -2231,6 +2268,7 @@ msc_status fp64_recover(msc_plan *p, const std::vector<int> &failed, const std::
     // right-hand sides and initial guesses: the parent's rows of each system
     const size_t vs = (size_t)c->R * n;
     MSC_CUDA(c->X0.alloc(vs));
+    MSC_CUDA(cudaStreamSynchronize(0));
     cudaStream_t cs = c->stream;
     for (int k = 0; k < nf; ++k) {
         const int s = failed[k];
@@ -2309,14 +2347,19 @@ msc_status msc_plan_create(msc_plan **plan, const msc_plan_desc *desc)
     if (desc->flags & 16) p->dcgs = false;     // classical Gram-Schmidt, two passes (CGS2)
     if (desc->flags & 32) p->gs = true;        // block Gauss-Seidel preconditioner M = L^-1
     p->sys.resize(p->B);
-    msc_status st = set_kernel_attributes(p->n, 0);
+    msc_status st = set_kernel_attributes();
     if (st != MSC_OK) { delete p; return st; }
-    cudaError_t e = cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMallocHost(&p->counter_host, sizeof(int));
+    // pinned block: the counter, the results and the cycle's step counts
+    const size_t o_report = 64, o_kcyc = o_report + (size_t)(p->B + 1) * sizeof(msc::SolveReport);
+    cudaError_t e = kit_acquire(o_kcyc + (size_t)p->B * sizeof(int), &p->kit);
     if (e != cudaSuccess) {
         delete p;
         return fail(MSC_ERR_CUDA, std::string("plan create: ") + cudaGetErrorString(e));
     }
+    p->stream = p->kit.stream;
+    p->counter_host = reinterpret_cast<int *>(p->kit.pinned);
+    p->report_host = reinterpret_cast<msc::SolveReport *>(p->kit.pinned + o_report);
+    p->kcyc_host = reinterpret_cast<int *>(p->kit.pinned + o_kcyc);
     *plan = p;
     return MSC_OK;
 }
@@ -2338,6 +2381,18 @@ msc_status msc_release_cached_memory(void)
     MSC_CUDA(plan_pool(&pool));
     MSC_CUDA(cudaDeviceSynchronize());
     MSC_CUDA(cudaMemPoolTrimTo(pool, 0));
+    int dev = -1;
+    MSC_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(g_kit_mutex);
+    auto &kits = idle_kits();
+    for (size_t i = 0; i < kits.size();) {
+        if (kits[i].dev == dev) {
+            kit_free(kits[i]);
+            kits.erase(kits.begin() + i);
+        } else {
+            ++i;
+        }
+    }
     return MSC_OK;
 }
 
@@ -2512,8 +2567,12 @@ msc_status msc_solve(msc_plan *p, double *psi_out, double *intensities_out, msc_
     if (st != MSC_OK) return st;
     cudaStream_t user = reinterpret_cast<cudaStream_t>(stream);
     cudaStream_t ps = p->stream;
-    cudaEvent_t ev;
-    MSC_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    struct Event {
+        cudaEvent_t e = nullptr;
+        ~Event() { if (e) cudaEventDestroy(e); }
+        operator cudaEvent_t() const { return e; }
+    } ev;
+    MSC_CUDA(cudaEventCreateWithFlags(&ev.e, cudaEventDisableTiming));
     MSC_CUDA(cudaEventRecord(ev, user));
     MSC_CUDA(cudaStreamWaitEvent(ps, ev, 0));
     // reset state (x = the warm-start guess when one is set, else 0)
@@ -2522,58 +2581,66 @@ msc_status msc_solve(msc_plan *p, double *psi_out, double *intensities_out, msc_
         MSC_CUDA(cudaMemcpyAsync(p->X.p, p->X0.p, vs * sizeof(double2), cudaMemcpyDeviceToDevice, ps));
     else
         MSC_CUDA(cudaMemsetAsync(p->X.p, 0, vs * sizeof(double2), ps));
-    MSC_CUDA(cudaMemsetAsync(p->iters.p, 0, p->B * sizeof(int), ps));
-    MSC_CUDA(cudaMemsetAsync(p->projv.p, 0, p->B * sizeof(int), ps));
-    MSC_CUDA(cudaMemsetAsync(p->cycles.p, 0, p->B * sizeof(int), ps));
-    MSC_CUDA(cudaMemsetAsync(p->status.p, 0, p->B * sizeof(int), ps));
-    MSC_CUDA(cudaMemsetAsync(p->kcyc.p, 0, p->B * sizeof(int), ps));
-    {
-        std::vector<int> ones(p->B, 1);
-        MSC_CUDA(cudaMemcpyAsync(p->unfinished.p, ones.data(), p->B * sizeof(int),
-                                 cudaMemcpyHostToDevice, ps));
-        MSC_CUDA(cudaStreamSynchronize(ps));
-    }
+    msc::k_solve_init<<<sys_blocks(p->B), 128, 0, ps>>>(p->state(), p->B);
+    // The first cycle's start runs as plain launches (r = b when x = 0: no residual
+    // product); from a zero guess there is nothing to look at before the first cycle.
     const int max_cycles = p->desc.max_iterations + 2;
-    int cycle = 0;
-    int64_t launches = 0;
-    bool pending = false;
-    for (; cycle < max_cycles; ++cycle) {
-        const bool x_zero = cycle == 0 && !p->has_x0;
-        MSC_CUDA(cudaGraphLaunch(x_zero ? p->g_start0 : p->g_start, ps));
-        launches += x_zero ? p->launches_start0 : p->launches_start;
+    const bool x_zero = !p->has_x0;
+    record_cycle_start_t(p, x_zero, ps);
+    MSC_CUDA(cudaGetLastError());
+    int64_t launches = 1 + cycle_start_launches(x_zero);
+    bool live = true;
+    if (!x_zero) {
         MSC_CUDA(cudaStreamSynchronize(ps));
-        if (pending && p->timing) accumulate_timing(p);
-        pending = false;
-        if (*p->counter_host == 0) break;
-        MSC_CUDA(cudaGraphLaunch(p->g_iter, ps));
-        launches += p->launches_iter;
-        pending = true;
+        live = *p->counter_host != 0;
+    }
+    int cycle = 0;
+    for (; live && cycle < max_cycles; ++cycle) {
+        MSC_CUDA(cudaGraphLaunch(p->g_cycle, ps));
+        launches += p->launches_cycle;
+        MSC_CUDA(cudaStreamSynchronize(ps));
+        if (p->timing) accumulate_timing(p);
+        live = *p->counter_host != 0;
     }
     p->launches_last = launches;
     p->cycles_last = cycle;
+    // results: one kernel gathers them, one copy brings them; the caller's outputs follow
+    // (again after an FP64 recovery)
+    auto write_outputs = [&]() -> msc_status {
+        if (psi_out)
+            MSC_CUDA(cudaMemcpyAsync(psi_out, p->X.p, vs * sizeof(double2), cudaMemcpyDeviceToDevice, ps));
+        if (intensities_out) {
+            msc::k_intensities<<<(p->R + 255) / 256, 256, 0, ps>>>(
+                p->R, 0, p->n, p->row_sys.p, p->sys_spec_row.p, p->sys_aspec.p, p->row_b.p, p->X.p,
+                intensities_out);
+            MSC_CUDA(cudaGetLastError());
+        }
+        return MSC_OK;
+    };
+    msc::k_solve_report<<<sys_blocks(p->B + 1), 128, 0, ps>>>(p->state(), p->B, p->use_tc ? p->tc_error.p : nullptr,
+                                                              p->wait_error.p, p->report.p);
     MSC_CUDA(cudaGetLastError());
-    if (p->use_tc) {
-        int tc_err = 0;
-        MSC_CUDA(cudaMemcpy(&tc_err, p->tc_error.p, sizeof(int), cudaMemcpyDeviceToHost));
-        if (tc_err) return fail(MSC_ERR_CUDA, "tensor-core block inverse timed out on an mbarrier wait");
-    }
-    {
-        int w_err = 0;
-        MSC_CUDA(cudaMemcpy(&w_err, p->wait_error.p, sizeof(int), cudaMemcpyDeviceToHost));
-        if (w_err) return fail(MSC_ERR_CUDA, "a bulk-copy wait of the streamed Arnoldi passes timed out");
-    }
-    std::vector<int> iters(p->B), cycles(p->B), status(p->B), unfinished(p->B), fallback(p->B, 0);
-    std::vector<int> projv(p->B);
-    std::vector<double> resid(p->B);
-    MSC_CUDA(cudaMemcpyAsync(iters.data(), p->iters.p, p->B * sizeof(int), cudaMemcpyDeviceToHost, ps));
-    MSC_CUDA(cudaMemcpyAsync(projv.data(), p->projv.p, p->B * sizeof(int), cudaMemcpyDeviceToHost, ps));
-    MSC_CUDA(cudaMemcpyAsync(cycles.data(), p->cycles.p, p->B * sizeof(int), cudaMemcpyDeviceToHost, ps));
-    MSC_CUDA(cudaMemcpyAsync(status.data(), p->status.p, p->B * sizeof(int), cudaMemcpyDeviceToHost, ps));
-    MSC_CUDA(cudaMemcpyAsync(unfinished.data(), p->unfinished.p, p->B * sizeof(int), cudaMemcpyDeviceToHost, ps));
-    MSC_CUDA(cudaMemcpyAsync(resid.data(), p->resid.p, p->B * sizeof(double), cudaMemcpyDeviceToHost, ps));
+    MSC_CUDA(cudaMemcpyAsync(p->report_host, p->report.p, (size_t)(p->B + 1) * sizeof(msc::SolveReport),
+                             cudaMemcpyDeviceToHost, ps));
+    st = write_outputs();
+    if (st != MSC_OK) return st;
+    MSC_CUDA(cudaEventRecord(ev, ps));
+    MSC_CUDA(cudaStreamWaitEvent(user, ev, 0));
     MSC_CUDA(cudaStreamSynchronize(ps));
-    for (int s = 0; s < p->B; ++s)
-        if (unfinished[s]) status[s] = MSC_ERR_NOT_CONVERGED;
+    if (p->report_host[p->B].status)
+        return fail(MSC_ERR_CUDA, "tensor-core block inverse timed out on an mbarrier wait");
+    if (p->report_host[p->B].unfinished)
+        return fail(MSC_ERR_CUDA, "a bulk-copy wait of the streamed Arnoldi passes timed out");
+    std::vector<int> iters(p->B), cycles(p->B), status(p->B), fallback(p->B, 0), projv(p->B);
+    std::vector<double> resid(p->B);
+    for (int s = 0; s < p->B; ++s) {
+        const msc::SolveReport &r = p->report_host[s];
+        iters[s] = r.iters;
+        projv[s] = r.projv;
+        cycles[s] = r.cycles;
+        status[s] = r.unfinished ? (int)MSC_ERR_NOT_CONVERGED : r.status;
+        resid[s] = r.resid;
+    }
     p->fallbacks_last = 0;
     if (p->mixed && !(p->desc.flags & 8)) {
         std::vector<int> failed;
@@ -2582,10 +2649,7 @@ msc_status msc_solve(msc_plan *p, double *psi_out, double *intensities_out, msc_
         if (!failed.empty()) {
             std::vector<msc_result> rec;
             msc_status rst = fp64_recover(p, failed, status, rec);
-            if (rst != MSC_OK) {
-                cudaEventDestroy(ev);
-                return rst;
-            }
+            if (rst != MSC_OK) return rst;
             for (size_t k = 0; k < failed.size(); ++k) {
                 const int s = failed[k];
                 iters[s] += rec[k].iterations;
@@ -2596,20 +2660,13 @@ msc_status msc_solve(msc_plan *p, double *psi_out, double *intensities_out, msc_
                 fallback[s] = 1;
             }
             p->fallbacks_last = (int)failed.size();
+            st = write_outputs();
+            if (st != MSC_OK) return st;
+            MSC_CUDA(cudaEventRecord(ev, ps));
+            MSC_CUDA(cudaStreamWaitEvent(user, ev, 0));
+            MSC_CUDA(cudaStreamSynchronize(ps));
         }
     }
-    if (psi_out)
-        MSC_CUDA(cudaMemcpyAsync(psi_out, p->X.p, vs * sizeof(double2), cudaMemcpyDeviceToDevice, ps));
-    if (intensities_out) {
-        msc::k_intensities<<<(p->R + 255) / 256, 256, 0, ps>>>(
-            p->R, 0, p->n, p->row_sys.p, p->sys_spec_row.p, p->sys_aspec.p, p->row_b.p, p->X.p,
-            intensities_out);
-        MSC_CUDA(cudaGetLastError());
-    }
-    MSC_CUDA(cudaEventRecord(ev, ps));
-    MSC_CUDA(cudaStreamWaitEvent(user, ev, 0));
-    MSC_CUDA(cudaStreamSynchronize(ps));
-    cudaEventDestroy(ev);
     msc_status worst = MSC_OK;
     for (int s = 0; s < p->B; ++s) {
         const int sst = status[s];
@@ -2647,12 +2704,16 @@ msc_status msc_plan_set_kernel_timing(msc_plan *p, int enable)
     if (st != MSC_OK) return st;
     const bool want = enable != 0;
     if (want == p->timing) return MSC_OK;
+    if (want && p->tev.empty()) {
+        p->tev.resize((size_t)msc_plan::kKinds * (p->m + 1) * 2);
+        for (cudaEvent_t &e : p->tev) MSC_CUDA(cudaEventCreate(&e));
+    }
     p->timing = want;
     for (int k = 0; k < msc_plan::kKinds; ++k) {
         p->t_ms[k] = 0.0;
         p->t_launches[k] = 0;
     }
-    return capture(p, record_cycle_iterations, &p->g_iter, &p->launches_iter);
+    return capture(p, record_cycle, &p->g_cycle, &p->launches_cycle);
 }
 
 msc_status msc_plan_kernel_timing(msc_plan *p, double *ms, int64_t *launches)
@@ -2812,7 +2873,10 @@ msc_status msc_plan_set_initial_guess(msc_plan *p, const double *psi0, int32_t o
         return MSC_OK;
     }
     const size_t vs = (size_t)p->R * p->n;
-    if (!p->X0.p) MSC_CUDA(p->X0.alloc(vs));
+    if (!p->X0.p) {
+        MSC_CUDA(p->X0.alloc(vs));
+        MSC_CUDA(cudaStreamSynchronize(0));
+    }
     cudaStream_t us = reinterpret_cast<cudaStream_t>(stream);
     MSC_CUDA(cudaMemcpyAsync(p->X0.p, psi0, vs * sizeof(double2),
                              on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, us));
@@ -2855,6 +2919,7 @@ msc_status msc_plan_set_adjoint(msc_plan *p, int32_t adjoint)
         for (size_t i = 0; i < rc.size(); ++i) c32[i] = make_float2((float)rc[i].x, (float)rc[i].y);
         MSC_CUDA(refill(p->row_c32, c32));
     }
+    MSC_CUDA(cudaStreamSynchronize(0));   // the new operator is in place for the plan's stream
     p->adjoint = want;
     return MSC_OK;
 }
@@ -2975,19 +3040,15 @@ int msc_run_multiscat(int gmres_preconditioner_flag, int convergence_significant
     if (st == MSC_OK)
         st = msc_plan_set_system(p, 0, C, ix.data(), iy.data(), perpendicular_kinetic_difference,
                                  wave_b, wave_c, 0, wave_a);
-    double *psi_dev = nullptr;
     msc_result res{};
-    if (st == MSC_OK) {
-        if (cudaMalloc(&psi_dev, (size_t)C * nz * sizeof(double2)) != cudaSuccess) st = MSC_ERR_CUDA;
-    }
-    if (st == MSC_OK) st = msc_solve(p, psi_dev, nullptr, &res, nullptr);
+    if (st == MSC_OK) st = msc_solve(p, nullptr, nullptr, &res, nullptr);
     if (st == MSC_OK || st == MSC_ERR_NOT_CONVERGED) {
-        if (cudaMemcpy(scattered_state_out, psi_dev, (size_t)C * nz * sizeof(double2),
+        // the plan's own solution vector (msc_solve has waited for it)
+        if (cudaMemcpy(scattered_state_out, p->X.p, (size_t)C * nz * sizeof(double2),
                        cudaMemcpyDeviceToHost) != cudaSuccess)
             st = MSC_ERR_CUDA;
     }
     if (iterations_out) *iterations_out = res.iterations;
-    if (psi_dev) cudaFree(psi_dev);
     msc_plan_destroy(p);
     return st;
 }
@@ -3126,7 +3187,7 @@ msc_status noalloc_scratch(unsigned char **out)
         cudaError_t e = cudaGetSymbolAddress(&ptr, g_noalloc_scratch);
         if (e != cudaSuccess || ptr == nullptr)
             return fail(MSC_ERR_CUDA, std::string("cudaGetSymbolAddress(scratch): ") + cudaGetErrorString(e));
-        msc_status st = set_kernel_attributes(0, 0);
+        msc_status st = set_kernel_attributes();
         if (st != MSC_OK) return st;
         g_noalloc_base[dev] = ptr;
     }

@@ -235,6 +235,19 @@ __device__ __forceinline__ uint32_t kmaj_off(int c, int k, int rows)
     return (uint32_t)(((k >> 3) * (rows >> 3) + (c >> 3)) * 128 + (c & 7) * 16 + (k & 7) * 2);
 }
 
+// BF16 hi / lo image of E (zero padded to kp x kp): [hi|lo][z/8][k/8][z%8][k%8].
+__global__ void k_resident_image(int n, int kp, const double *__restrict__ E, __nv_bfloat16 *__restrict__ img)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= kp * kp) return;
+    const int z = i / kp, k = i - z * kp;
+    const double v = z < n && k < n ? E[(size_t)z * n + k] : 0.0;
+    const __nv_bfloat16 hi = __float2bfloat16_rn((float)v);
+    const size_t off = ((size_t)(z / 8) * (kp / 8) + k / 8) * 64 + (z % 8) * 8 + k % 8;
+    img[off] = hi;
+    img[(size_t)kp * kp + off] = __float2bfloat16_rn((float)(v - (double)__bfloat162float(hi)));
+}
+
 // G = 1: the CTA's 16 warps work on one tile at a time.  G = 2: two groups
 // of 8 warps (warps 0-7, 8-15), each with its own B buffer, TMEM columns,
 // mbarrier and named barrier, run independent tile loops over the shared E

@@ -41,6 +41,26 @@ __host__ __device__ constexpr size_t stream_smem(int kp, int N, int S)
     return S * stream_stage_bytes(kp) + (size_t)4 * N * kp + 1024;
 }
 
+// The two images: one contiguous piece [hi, lo][2 K blocks][kp / 8][8 z][8 k] per 16
+// of K, K = z in zk (E^T x) and K = k in kz (E y); zero past n.
+__global__ void k_stream_images(int n, int kp, const double *__restrict__ E, __nv_bfloat16 *__restrict__ zk,
+                                __nv_bfloat16 *__restrict__ kz)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= kp * kp) return;
+    const int z = i / kp, k = i - z * kp, kb = kp / 8;
+    const double v = z < n && k < n ? E[(size_t)z * n + k] : 0.0;
+    const __nv_bfloat16 hi = __float2bfloat16_rn((float)v);
+    const __nv_bfloat16 lo = __float2bfloat16_rn((float)(v - (double)__bfloat162float(hi)));
+    const size_t part = (size_t)16 * kp, in = (size_t)(z % 8) * 8 + k % 8;
+    const size_t a = (size_t)(z / 16) * 2 * part + ((size_t)(z / 8 % 2) * kb + k / 8) * 64 + in;
+    const size_t b = (size_t)(k / 16) * 2 * part + ((size_t)(k / 8 % 2) * kb + z / 8) * 64 + in;
+    zk[a] = hi;
+    zk[a + part] = lo;
+    kz[b] = hi;
+    kz[b + part] = lo;
+}
+
 struct TcStreamParams {
     TcParams t;                          // e_img unused
     const __nv_bfloat16 *img1, *img2;    // [piece][hi, lo][2 K blocks][kp / 8][8][8]
