@@ -1060,20 +1060,47 @@ __device__ void arnoldi_givens(GmresState &st, int s, int m, int j, double rtol,
     if (stop) st.active[s] = 0;
 }
 
-// y = R^-1 g over the kcyc columns of this cycle.
-__global__ void k_trisolve(GmresState st, int nsys, int m)
+// y = R^-1 g over the kcyc columns of this cycle: one warp per system, column by
+// column (lane l holds rows l and l + 32 of g), the next column on its way while
+// one is applied.  (One thread per system walked k^2 / 2 dependent loads: 60 us for
+// 30 columns; 4 us now.)
+__global__ void __launch_bounds__(32) k_trisolve(GmresState st, int m)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nsys) return;
+    const int s = blockIdx.x, lane = threadIdx.x;
     const int k = st.kcyc[s];
     if (k == 0) return;
     const double2 *H = st.H + (size_t)s * (m + 1) * m;
     const double2 *g = st.g + (size_t)s * (m + 1);
     double2 *y = st.y + (size_t)s * m;
+    const double2 zero = make_double2(0.0, 0.0), one = make_double2(1.0, 0.0);
+    double2 gv[2], inv[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int l = lane + 32 * h;
+        gv[h] = l < k ? g[l] : zero;
+        inv[h] = l < k ? cdiv(one, H[(size_t)l * (m + 1) + l]) : zero;
+    }
+    auto column = [&](int i, double2 (&c)[2]) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int l = lane + 32 * h;
+            c[h] = i >= 0 && l < i ? H[(size_t)i * (m + 1) + l] : zero;
+        }
+    };
+    double2 cur[2], nxt[2];
+    column(k - 1, cur);
     for (int i = k - 1; i >= 0; --i) {
-        double2 acc = g[i];
-        for (int l = i + 1; l < k; ++l) acc = csub(acc, cmul(H[(size_t)l * (m + 1) + i], y[l]));
-        y[i] = cdiv(acc, H[(size_t)i * (m + 1) + i]);
+        column(i - 1, nxt);
+        const double2 own = i < 32 ? cmul(gv[0], inv[0]) : cmul(gv[1], inv[1]);
+        double2 yi;
+        yi.x = __shfl_sync(0xffffffffu, own.x, i & 31);
+        yi.y = __shfl_sync(0xffffffffu, own.y, i & 31);
+        if (lane == (i & 31)) y[i] = yi;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            gv[h] = csub(gv[h], cmul(cur[h], yi));
+            cur[h] = nxt[h];
+        }
     }
 }
 
@@ -1108,8 +1135,13 @@ __device__ __forceinline__ void elem_range(const ArnoldiArgs &a, int tile, int s
     ne = min(tot, lo + per) - lo;
 }
 
-// Last-arriving block of system s sums the system's partials into dst[0..nslot).
-__device__ __forceinline__ bool last_block_reduce(const ArnoldiArgs &a, int s, int nslot, double2 *dst)
+// Last-arriving block of system s sums the system's partials into dst[0..nslot), in a
+// fixed order.  Up to 8 slots: a warp per slot, lanes over the blocks.  More: thread
+// groups of one slot per thread (consecutive slots: coalesced rows of the partial
+// array) take every G-th block, the groups' sums add up in shared memory (gsum: 256
+// entries, the caller's scratch).  256 threads.
+__device__ __forceinline__ bool last_block_reduce(const ArnoldiArgs &a, int s, int nslot, double2 *dst,
+                                                  double2 *gsum)
 {
     __shared__ int is_last;
     __threadfence();
@@ -1124,20 +1156,54 @@ __device__ __forceinline__ bool last_block_reduce(const ArnoldiArgs &a, int s, i
     if (!is_last) return false;
     __threadfence();
     const int b0 = a.sys_tile0[s] * a.split, b1 = a.sys_tile0[s + 1] * a.split;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int i = warp; i < nslot; i += (blockDim.x >> 5)) {
-        double sr = 0.0, si = 0.0;
-        for (int b = b0 + lane; b < b1; b += 32) {
-            const double2 v = __ldcg(a.partial + (size_t)b * a.pstride + i);
-            sr += v.x;
-            si += v.y;
+    if (nslot <= 8) {
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        if (warp < nslot) {
+            double2 v = make_double2(0.0, 0.0);
+#pragma unroll 4
+            for (int b = b0 + lane; b < b1; b += 32) v = cadd(v, __ldcg(a.partial + (size_t)b * a.pstride + warp));
+            v.x = warp_sum(v.x);
+            v.y = warp_sum(v.y);
+            if (lane == 0) dst[warp] = v;
         }
-        sr = warp_sum(sr);
-        si = warp_sum(si);
-        if (lane == 0) dst[i] = make_double2(sr, si);
+        __syncthreads();
+        return true;
+    }
+    int P = 16;
+    while (P < nslot && P < 256) P *= 2;
+    const int G = 256 / P, slot = threadIdx.x & (P - 1), g = threadIdx.x / P;
+    double2 acc = make_double2(0.0, 0.0);
+    if (slot < nslot) {
+        const double2 *pp = a.partial + slot;
+#pragma unroll 8
+        for (int b = b0 + g; b < b1; b += G) acc = cadd(acc, __ldcg(pp + (size_t)b * a.pstride));
+    }
+    gsum[threadIdx.x] = acc;
+    __syncthreads();
+    if (threadIdx.x < P && slot < nslot) {
+        for (int q = 1; q < G; ++q) acc = cadd(acc, gsum[q * P + slot]);
+        dst[slot] = acc;
     }
     __syncthreads();
     return true;
+}
+
+// Sums of four values over the warp: every lane of group lane / 8 returns the total of
+// value lane / 8 (6 exchanges instead of 20, in a fixed order).
+__device__ __forceinline__ double warp_sum4(double a, double b, double c, double d, int lane)
+{
+    const bool up = lane & 16;
+    double p = up ? c : a, q = up ? d : b;
+    const double sp = up ? a : c, sq = up ? b : d;
+    p += __shfl_xor_sync(0xffffffffu, sp, 16);
+    q += __shfl_xor_sync(0xffffffffu, sq, 16);
+    const bool hi = lane & 8;
+    double r = hi ? q : p;
+    r += __shfl_xor_sync(0xffffffffu, hi ? p : q, 8);
+    r += __shfl_xor_sync(0xffffffffu, r, 4);
+    r += __shfl_xor_sync(0xffffffffu, r, 2);
+    r += __shfl_xor_sync(0xffffffffu, r, 1);
+    return r;
 }
 
 // P1: h1 = Q^H w.  Warps take (basis vector, sub-range) tasks: each vector's
@@ -1219,7 +1285,7 @@ k_arnoldi_p1(ArnoldiArgs a, const typename CT<R>::t *__restrict__ Q, int nvec,
         }
         out[i] = acc;
     }
-    last_block_reduce(a, s, nvec, h1 + (size_t)s * hstride);
+    last_block_reduce(a, s, nvec, h1 + (size_t)s * hstride, &red[0][0]);
 }
 
 __device__ void arnoldi_givens(GmresState &st, int s, int m, int j, double rtol, int max_iter,
@@ -1315,7 +1381,8 @@ k_arnoldi_p2(ArnoldiArgs a, const typename CT<R>::t *__restrict__ Q, int nvec,
             if (lane == 0) out[task] = make_double2(sr, norm ? 0.0 : si);
         }
     }
-    if (last_block_reduce(a, s, nvec + 1, st.h2 + (size_t)s * hs)) {
+    __shared__ double2 gsum[256];
+    if (last_block_reduce(a, s, nvec + 1, st.h2 + (size_t)s * hs, gsum)) {
         if (threadIdx.x == 0) arnoldi_givens(st, s, m, j, rtol, max_iter, inner_rtol, cgs2 != 0);
     }
 }
@@ -1350,7 +1417,7 @@ k_arnoldi_p2(ArnoldiArgs a, const typename CT<R>::t *__restrict__ Q, int nvec,
 struct DcgsState {
     double2 *Hraw;    // [B][(m+1)*m]  unrotated Hessenberg (column j at j*(m+1))
     double2 *dsum;    // [B][2(m+1)]   per-system reduction results of the step
-    double2 *coef;    // [B][cstride]  update coefficients (see dcgs_coefficients_p)
+    double2 *coef;    // [B][cstride]  update coefficients (see dcgs_coefficients_block)
     double2 *gsave;   // [B]           g[j] before the provisional rotation j
     int cstride;      // 2 m + 4
 };
@@ -1364,16 +1431,16 @@ struct DcgsState {
 __device__ double dcgs_rotate_column_p(const double2 *raw, double2 *H, double2 *cs, double2 *sn,
                                        double2 *g, double2 gj, int j)
 {
-    for (int i = 0; i <= j + 1; ++i) H[i] = raw[i];
+    // the entry a rotation passes on to the next one stays in a register
+    double2 a = raw[0];
+#pragma unroll 4
     for (int i = 0; i < j; ++i) {
         const double c = cs[i].x;
-        const double2 sv = sn[i];
-        const double2 a = H[i], b = H[i + 1];
+        const double2 sv = sn[i], b = raw[i + 1];
         H[i] = cadd(cscale(a, c), cmul(sv, b));
-        H[i + 1] = csub(cscale(b, c), cmul(cconj(sv), a));
+        a = csub(cscale(b, c), cmul(cconj(sv), a));
     }
-    const double2 a = H[j];
-    const double beta = H[j + 1].x;            // real, >= 0 (a norm)
+    const double beta = raw[j + 1].x;          // real, >= 0 (a norm)
     const double aa = sqrt(cabs2(a));
     const double r = hypot(aa, beta);
     double c;
@@ -1397,75 +1464,10 @@ __device__ double dcgs_rotate_column_p(const double2 *raw, double2 *H, double2 *
     return sqrt(cabs2(g[j + 1]));
 }
 
-__device__ __forceinline__ double dcgs_rotate_column(GmresState &st, const DcgsState &ds, int s, int m, int j)
-{
-    return dcgs_rotate_column_p(ds.Hraw + (size_t)s * (m + 1) * m + (size_t)j * (m + 1),
-                                st.H + (size_t)s * (m + 1) * m + (size_t)j * (m + 1),
-                                st.cs + (size_t)s * m, st.sn + (size_t)s * m,
-                                st.g + (size_t)s * (m + 1), ds.gsave[s], j);
-}
-
 __device__ __forceinline__ bool dcgs_stop(const GmresState &st, int s, double est, double rtol,
                                           double inner_rtol)
 {
     return !isfinite(est) || est <= fmax(rtol * st.bnorm[s], inner_rtol * st.beta0[s]);
-}
-
-// Per-system scalar work of the reduction (one thread): finalise column j-1,
-// redo its rotation, form h_j and the update coefficients:
-//   coef[0..j)        a_i = -s_i / nu            (q_j = v / nu + sum a_i Q_i)
-//   coef[j+1 .. 2j+1) b_i = -(c_i - s_i d / nu)  (v_{j+1} = w / nu - (d / nu) v + sum b_i Q_i)
-//   coef[2m+2] = (1 / nu, 0), coef[2m+3] = -d / nu
-// on one system's arrays (global or shared memory): raw = its unrotated
-// Hessenberg columns, sum = its reduction results, Hj1 = its column j - 1 of
-// H, hs = scratch of j + 1 entries.  Returns 1 when the system stops
-// (converged, or no new direction), with *est set when j > 0.
-__device__ int dcgs_coefficients_p(double2 *raw, const double2 *sum, double2 *Hj1, double2 *cs,
-                                   double2 *sn, double2 *g, double2 gsave, double2 *cf, double2 *hs,
-                                   int m, int j, double bnorm, double beta0, double rtol,
-                                   double inner_rtol, double *est)
-{
-    const double2 *sv = sum;               // s_i = q_i^H v, i < j;  sum[j] = ||v||^2
-    const double2 *tv = sum + (j + 1);     // t_i = q_i^H w, i < j;  tv[j] = v^H w
-    double ss = 0.0;
-    for (int i = 0; i < j; ++i) ss += cabs2(sv[i]);
-    const double nu2 = sum[j].x - ss;
-    const double nu = sqrt(fmax(nu2, 0.0));
-    if (j == 0) {
-        // v = q_0 up to rounding; g[0] = beta follows q_0 = v / nu
-        g[0] = cscale(g[0], nu);
-    } else {
-        double2 *col = raw + (size_t)(j - 1) * (m + 1);
-        for (int i = 0; i < j; ++i) col[i] = cadd(col[i], sv[i]);
-        col[j] = make_double2(nu, 0.0);
-        *est = dcgs_rotate_column_p(col, Hj1, cs, sn, g, gsave, j - 1);
-        if (!isfinite(*est) || *est <= fmax(rtol * bnorm, inner_rtol * beta0))
-            return 1;                      // q_0 .. q_{j-1} are final; kcyc = j
-    }
-    if (!(nu > 1e-300) || !isfinite(nu)) return 1;
-    const double inu = 1.0 / nu;
-    // Hs = Hbar[:j+1, :j] s (column k has entries 0..k+1)
-    for (int i = 0; i <= j; ++i) hs[i] = make_double2(0.0, 0.0);
-    for (int k = 0; k < j; ++k) {
-        const double2 *colk = raw + (size_t)k * (m + 1);
-        for (int i = 0; i <= k + 1; ++i) hs[i] = cadd(hs[i], cmul(colk[i], sv[k]));
-    }
-    double2 sht = make_double2(0.0, 0.0);   // s^H t
-    for (int i = 0; i < j; ++i) sht = cadd(sht, cmul(cconj(sv[i]), tv[i]));
-    double2 *colj = raw + (size_t)j * (m + 1);
-    for (int i = 0; i < j; ++i) colj[i] = cscale(csub(tv[i], hs[i]), inu);
-    colj[j] = cscale(csub(cscale(csub(tv[j], sht), inu), hs[j]), inu);
-    const double2 d = cadd(cscale(hs[j], inu), colj[j]);
-    const double2 dn = cscale(d, inu);
-    for (int i = 0; i < j; ++i) {
-        const double2 ci = cadd(cscale(hs[i], inu), colj[i]);
-        cf[i] = cscale(sv[i], -inu);
-        cf[j + 1 + i] = make_double2(-(ci.x - (sv[i].x * dn.x - sv[i].y * dn.y)),
-                                     -(ci.y - (sv[i].x * dn.y + sv[i].y * dn.x)));
-    }
-    cf[2 * m + 2] = make_double2(inu, 0.0);
-    cf[2 * m + 3] = make_double2(-dn.x, -dn.y);
-    return 0;
 }
 
 // Double2 entries of the shared scratch dcgs_coefficients_block needs.
@@ -1474,13 +1476,19 @@ __host__ __device__ constexpr int dcgs_block_scratch(int m)
     return (m + 1) * (m + 1) + 5 * (m + 1) + 4 * m + 4;
 }
 
-// dcgs_coefficients_p for the last block of a system: the whole block copies
-// the system's Hessenberg columns 0..j, reduction results, rotations and g
-// into shared memory (one round of parallel loads), thread 0 runs the
-// serial algebra there, and the block writes back what changed.  The
-// serial part then waits on shared memory instead of an L2 round trip per
-// element (the tail of the reduction kernel).  sc: dcgs_block_scratch(m)
-// entries of shared memory.
+// Per-system scalar work of the reduction, by the last block of a system (256
+// threads): finalise column j-1, redo its rotation, form h_j and the update
+// coefficients:
+//   coef[0..j)        a_i = -s_i / nu            (q_j = v / nu + sum a_i Q_i)
+//   coef[j+1 .. 2j+1) b_i = -(c_i - s_i d / nu)  (v_{j+1} = w / nu - (d / nu) v + sum b_i Q_i)
+//   coef[2m+2] = (1 / nu, 0), coef[2m+3] = -d / nu
+// The block stages the system's Hessenberg columns 0..j, reduction results,
+// rotations and g in shared memory (sc: dcgs_block_scratch(m) entries) and writes
+// back what changed.  Warp 0 runs the rotation of column j-1, a chain over its
+// entries, while the rows of Hs = Hbar s, one thread each, and s^H t are summed on
+// other warps: the chain is all that is left of the serial part (one thread did the
+// j^2 / 2 products of Hs before: 12 of the 28 us of a reduction at j = 20 on a
+// 121-row system).
 __device__ void dcgs_coefficients_block(GmresState &st, const DcgsState &ds, int s, int m, int j,
                                         double rtol, double inner_rtol, double2 *sc)
 {
@@ -1491,65 +1499,113 @@ __device__ void dcgs_coefficients_block(GmresState &st, const DcgsState &ds, int
     double2 *sn = cs + m;                        // [m]
     double2 *g = sn + m;                         // [M1]
     double2 *Hj1 = g + M1;                       // [M1] column j - 1 of H
-    double2 *cf = Hj1 + M1;                      // [2 m + 4]
-    double2 *hs = cf + 2 * m + 4;                // [M1]
-    __shared__ int res;
+    double2 *hs = Hj1 + M1;                      // [M1] Hs
+    __shared__ int stop_s;
+    __shared__ double nu_s;
+    __shared__ double2 sht_s, dn_s;
     const size_t hb = (size_t)s * M1 * m;
-    const int nt = blockDim.x;
-    for (int i = threadIdx.x; i < ncol * M1; i += nt) raw[i] = ds.Hraw[hb + i];
-    for (int i = threadIdx.x; i < 2 * M1; i += nt) sum[i] = ds.dsum[(size_t)s * 2 * M1 + i];
-    for (int i = threadIdx.x; i < m; i += nt) {
+    const int nt = blockDim.x, t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    for (int i = t; i < ncol * M1; i += nt) raw[i] = ds.Hraw[hb + i];
+    for (int i = t; i < 2 * M1; i += nt) sum[i] = ds.dsum[(size_t)s * 2 * M1 + i];
+    for (int i = t; i < m; i += nt) {
         cs[i] = st.cs[(size_t)s * m + i];
         sn[i] = st.sn[(size_t)s * m + i];
     }
-    for (int i = threadIdx.x; i < M1; i += nt) g[i] = st.g[(size_t)s * M1 + i];
+    for (int i = t; i < M1; i += nt) g[i] = st.g[(size_t)s * M1 + i];
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double est = 0.0;
-        res = dcgs_coefficients_p(raw, sum, Hj1, cs, sn, g, ds.gsave[s], cf, hs, m, j, st.bnorm[s],
-                                  st.beta0[s], rtol, inner_rtol, &est);
-        if (j > 0) st.est[s] = est;
-        if (res) st.active[s] = 0;
+    const double2 *sv = sum;               // s_i = q_i^H v, i < j;  sum[j] = ||v||^2
+    const double2 *tv = sum + (j + 1);     // t_i = q_i^H w, i < j;  tv[j] = v^H w
+    if (warp == 0) {
+        double ss = 0.0;
+        for (int i = lane; i < j; i += 32) ss += cabs2(sv[i]);
+        ss = warp_sum(ss);
+        if (lane == 0) nu_s = sqrt(fmax(sum[j].x - ss, 0.0));
+    } else if (warp == 1) {
+        double2 d = make_double2(0.0, 0.0);
+        for (int i = lane; i < j; i += 32) d = cadd(d, cmul(cconj(sv[i]), tv[i]));
+        d.x = warp_sum(d.x);
+        d.y = warp_sum(d.y);
+        if (lane == 0) sht_s = d;
+    }
+    __syncthreads();
+    const double nu = nu_s;
+    // column j - 1 becomes final
+    for (int i = t; i <= j && j > 0; i += nt) {
+        double2 &e = raw[(size_t)(j - 1) * M1 + i];
+        e = i < j ? cadd(e, sv[i]) : make_double2(nu, 0.0);
+    }
+    __syncthreads();
+    if (t == 0) {
+        int stop = !(nu > 1e-300) || !isfinite(nu);
+        if (j == 0) {
+            g[0] = cscale(g[0], nu);       // v = q_0 up to rounding; g[0] = beta follows q_0 = v / nu
+        } else {
+            const double est = dcgs_rotate_column_p(raw + (size_t)(j - 1) * M1, Hj1, cs, sn, g,
+                                                    ds.gsave[s], j - 1);
+            st.est[s] = est;
+            // q_0 .. q_{j-1} are final when the rotated column meets the bound; kcyc = j
+            if (!isfinite(est) || est <= fmax(rtol * st.bnorm[s], inner_rtol * st.beta0[s])) stop = 1;
+        }
+        if (stop) st.active[s] = 0;
+        stop_s = stop;
+    } else if (t >= 32 && t - 32 <= j) {
+        const int i = t - 32;              // Hs_i: column k has entries 0..k+1
+        double2 h = make_double2(0.0, 0.0);
+#pragma unroll 4
+        for (int k = max(i - 1, 0); k < j; ++k) h = cadd(h, cmul(raw[(size_t)k * M1 + i], sv[k]));
+        hs[i] = h;
     }
     __syncthreads();
     if (j == 0) {
-        if (threadIdx.x == 0) st.g[(size_t)s * M1] = g[0];
+        if (t == 0) st.g[(size_t)s * M1] = g[0];
     } else {
         // column j - 1: its final entries 0..j, its rotated form, rotation j - 1, g
-        for (int i = threadIdx.x; i <= j; i += nt) {
+        for (int i = t; i <= j; i += nt) {
             ds.Hraw[hb + (size_t)(j - 1) * M1 + i] = raw[(size_t)(j - 1) * M1 + i];
             st.H[hb + (size_t)(j - 1) * M1 + i] = Hj1[i];
         }
-        if (threadIdx.x == 0) {
+        if (t == 0) {
             st.cs[(size_t)s * m + j - 1] = cs[j - 1];
             st.sn[(size_t)s * m + j - 1] = sn[j - 1];
             st.g[(size_t)s * M1 + j - 1] = g[j - 1];
             st.g[(size_t)s * M1 + j] = g[j];
         }
     }
-    if (res == 0) {
-        double2 *cfg = ds.coef + (size_t)s * ds.cstride;
-        for (int i = threadIdx.x; i <= j; i += nt) ds.Hraw[hb + (size_t)j * M1 + i] = raw[(size_t)j * M1 + i];
-        for (int i = threadIdx.x; i < j; i += nt) {
-            cfg[i] = cf[i];
-            cfg[j + 1 + i] = cf[j + 1 + i];
+    if (stop_s) return;
+    const double inu = 1.0 / nu;
+    double2 *cfg = ds.coef + (size_t)s * ds.cstride;
+    double2 col = make_double2(0.0, 0.0);
+    if (t <= j) {
+        col = t < j ? cscale(csub(tv[t], hs[t]), inu)
+                    : cscale(csub(cscale(csub(tv[j], sht_s), inu), hs[j]), inu);
+        ds.Hraw[hb + (size_t)j * M1 + t] = col;
+        if (t == j) {
+            const double2 dn = cscale(cadd(cscale(hs[j], inu), col), inu);
+            dn_s = dn;
+            cfg[2 * m + 2] = make_double2(inu, 0.0);
+            cfg[2 * m + 3] = make_double2(-dn.x, -dn.y);
         }
-        if (threadIdx.x == 0) {
-            cfg[2 * m + 2] = cf[2 * m + 2];
-            cfg[2 * m + 3] = cf[2 * m + 3];
-        }
+    }
+    __syncthreads();
+    if (t < j) {
+        const double2 c = cadd(cscale(hs[t], inu), col), dn = dn_s;
+        cfg[t] = cscale(sv[t], -inu);
+        cfg[j + 1 + t] = make_double2(-(c.x - (sv[t].x * dn.x - sv[t].y * dn.y)),
+                                      -(c.y - (sv[t].x * dn.y + sv[t].y * dn.x)));
     }
 }
 
 template <typename R> struct DcgsUnroll { static constexpr int value = 8; };
 template <> struct DcgsUnroll<double> { static constexpr int value = 4; };
 
-// Reduction pass of step j over row chunks.  Each warp takes sub-ranges of
-// 32 U elements of the block's chunk, holds v and w there in registers and
-// streams q_0 .. q_{j-1} and v itself (the basis slots 0 .. j), two dots per
-// vector (q_i^H v, q_i^H w), reduced across the warp per vector and added in
-// a fixed order (deterministic).  The last block of a system reduces the
-// per-block partials and runs dcgs_coefficients_block.
+// Reduction pass of step j over row chunks.  A warp takes 32 U elements of the
+// block's chunk, holds v and w there in registers and streams basis vectors (slots
+// 0 .. j, slot j is v itself), two dots per vector (q_i^H v, q_i^H w).  A chunk of
+// fewer than 8 such pieces (a few rows: small batches, single systems) leaves warps
+// over: they split the vectors, every VG-th each, so that a 100-element chunk's
+// j + 1 vectors pass through 8 warps instead of one.  Sums across lanes, pieces and
+// blocks are added in a fixed order (deterministic).  The last block of a system
+// reduces the per-block partials and runs dcgs_coefficients_block.
 // Precision: a lane's products and its partial sum of U terms are formed in
 // the vectors' own type (FP32 for the inner solve of the mixed form: FP64
 // products there made the FP64 pipe, not memory, the limit), the sums across
@@ -1576,12 +1632,13 @@ k_dcgs_reduce(ArnoldiArgs a, const typename CT<R>::t *__restrict__ Q, int j,
     elem_range<R>(a, blk, 0, e0, ne);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nv = j + 1;                        // basis slots 0..j (slot j holds v)
-    for (int i = threadIdx.x; i < 2 * nv * NW; i += blockDim.x)
-        red[i / NW][i % NW] = make_double2(0.0, 0.0);
-    __syncthreads();
+    const int EG = min(NW, (ne + 32 * U - 1) / (32 * U));   // pieces of the chunk at a time
+    const int VG = NW / EG;                                  // warps sharing a piece's vectors
+    const int eg = warp % EG, vg = warp / EG;
     const C2 *vp = Q + (size_t)j * a.qstride + e0;
     const C2 *wp = W + e0;
-    for (int base = warp * 32 * U; base < ne; base += NW * 32 * U) {
+    bool first = true;
+    for (int base = eg * 32 * U; base < ne && vg < VG; base += EG * 32 * U) {
         C2 vv[U], ww[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -1592,23 +1649,20 @@ k_dcgs_reduce(ArnoldiArgs a, const typename CT<R>::t *__restrict__ Q, int j,
         // q_i is loaded one vector ahead, so its loads are in flight while
         // the previous vector's products and warp sums run
         C2 qn[U];
+        auto load = [&](int i) {
+            const C2 *q = Q + (size_t)i * a.qstride + e0;
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int e = base + u * 32 + lane;
-            qn[u] = (e < ne) ? Q[e0 + e] : mk2<R>(0, 0);
-        }
-        for (int i = 0; i < nv; ++i) {
+            for (int u = 0; u < U; ++u) {
+                const int e = base + u * 32 + lane;
+                qn[u] = (e < ne) ? q[e] : mk2<R>(0, 0);
+            }
+        };
+        if (vg < nv) load(vg);
+        for (int i = vg; i < nv; i += VG) {
             C2 qv[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) qv[u] = qn[u];
-            if (i + 1 < nv) {
-                const C2 *q = Q + (size_t)(i + 1) * a.qstride + e0;
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int e = base + u * 32 + lane;
-                    qn[u] = (e < ne) ? q[e] : mk2<R>(0, 0);
-                }
-            }
+            if (i + VG < nv) load(i + VG);
             // products and the lane's partial sum of U terms in the vectors'
             // own precision, the sums across lanes, warps and blocks in FP64
             R ar = 0, ai = 0, br = 0, bi = 0;
@@ -1620,27 +1674,27 @@ k_dcgs_reduce(ArnoldiArgs a, const typename CT<R>::t *__restrict__ Q, int j,
                 br = fma(qx, ww[u].x, fma(qy, ww[u].y, br));
                 bi = fma(qx, ww[u].y, fma(-qy, ww[u].x, bi));
             }
-            const double sar = warp_sum((double)ar), sai = warp_sum((double)ai);
-            const double sbr = warp_sum((double)br), sbi = warp_sum((double)bi);
-            if (lane == 0) {
-                double2 &x = red[i][warp];
-                double2 &y = red[nv + i][warp];
-                x.x += sar; x.y += sai;
-                y.x += sbr; y.y += sbi;
+            const double r = warp_sum4((double)ar, (double)ai, (double)br, (double)bi, lane);
+            if ((lane & 7) == 0) {
+                // lane 0, 8: q^H v (re, im); lane 16, 24: q^H w
+                double2 &x = red[(lane & 16) ? nv + i : i][eg];
+                double &c = (lane & 8) ? x.y : x.x;
+                c = first ? r : c + r;
             }
         }
+        first = false;
     }
     __syncthreads();
     double2 *out = a.partial + (size_t)blk * a.pstride;
     for (int i = threadIdx.x; i < 2 * nv; i += blockDim.x) {
         double2 acc = red[i][0];
-        for (int w = 1; w < NW; ++w) {
+        for (int w = 1; w < EG; ++w) {
             acc.x += red[i][w].x;
             acc.y += red[i][w].y;
         }
         out[i] = acc;
     }
-    if (last_block_reduce(a, s, 2 * nv, ds.dsum + (size_t)s * 2 * (m + 1))) {
+    if (last_block_reduce(a, s, 2 * nv, ds.dsum + (size_t)s * 2 * (m + 1), &red[0][0])) {
         extern __shared__ __align__(16) unsigned char dcgs_scratch[];   // dcgs_block_scratch(m) entries
         dcgs_coefficients_block(st, ds, s, m, j, rtol, inner_rtol, reinterpret_cast<double2 *>(dcgs_scratch));
     }
@@ -1733,11 +1787,10 @@ k_dcgs_reduce_bulk(ArnoldiArgs a, const float2 *__restrict__ Q, int j, const flo
         }
     };
     auto add_sums = [&](int i, float ar, float ai, float br, float bi) {
-        const double sar = warp_sum((double)ar), sai = warp_sum((double)ai);
-        const double sbr = warp_sum((double)br), sbi = warp_sum((double)bi);
-        if (lane == 0) {
-            red[i][warp] = make_double2(sar, sai);
-            red[nv + i][warp] = make_double2(sbr, sbi);
+        const double r = warp_sum4((double)ar, (double)ai, (double)br, (double)bi, lane);
+        if ((lane & 7) == 0) {
+            double2 &x = red[(lane & 16) ? nv + i : i][warp];
+            ((lane & 8) ? x.y : x.x) = r;
         }
     };
     bool ok = true;
@@ -1792,7 +1845,7 @@ k_dcgs_reduce_bulk(ArnoldiArgs a, const float2 *__restrict__ Q, int j, const flo
         }
         out[k] = acc;
     }
-    if (last_block_reduce(a, s, 2 * nv, ds.dsum + (size_t)s * 2 * (m + 1))) {
+    if (last_block_reduce(a, s, 2 * nv, ds.dsum + (size_t)s * 2 * (m + 1), &red[0][0])) {
         dcgs_coefficients_block(st, ds, s, m, j, rtol, inner_rtol, reinterpret_cast<double2 *>(smem_raw));
     }
 }
@@ -1851,14 +1904,16 @@ __device__ void dcgs_update_finish_block(GmresState &st, const DcgsState &ds, in
 // (one read of q_0 .. q_{j-1}, v, w; two writes), ||v_{j+1}||^2 reduced per
 // system; the last block forms the provisional column j and its rotation,
 // counts the iteration and applies the stop rules.
-template <typename R>
-__global__ void __launch_bounds__(256)
+// UQ basis vectors are loaded per batch: 4 and four blocks per SM where there are
+// blocks enough (memory-bound), 8 where a block has an SM to itself and waits for
+// its own loads.
+template <typename R, int UQ>
+__global__ void __launch_bounds__(256, UQ == 4 ? 4 : 2)
 k_dcgs_update(ArnoldiArgs a, typename CT<R>::t *__restrict__ Q, int j,
               const typename CT<R>::t *__restrict__ W, GmresState st, DcgsState ds, int m,
               double rtol, int max_iter, double inner_rtol)
 {
     using C2 = typename CT<R>::t;
-    constexpr int UQ = 4;                        // basis vectors loaded per batch
     __shared__ C2 ca[kMaxRestart], cb[kMaxRestart];
     __shared__ double wsum[8];
     const int blk = blockIdx.x;
@@ -1942,7 +1997,7 @@ k_dcgs_update(ArnoldiArgs a, typename CT<R>::t *__restrict__ Q, int j,
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += wsum[w];
         a.partial[(size_t)blk * a.pstride] = make_double2(t, 0.0);
     }
-    if (last_block_reduce(a, s, 1, st.h2 + (size_t)s * (m + 2))) {
+    if (last_block_reduce(a, s, 1, st.h2 + (size_t)s * (m + 2), nullptr)) {
         extern __shared__ __align__(16) unsigned char dcgs_scratch[];   // 3 (m + 1) + 2 m entries
         dcgs_update_finish_block(st, ds, s, m, j, rtol, max_iter, inner_rtol,
                                  reinterpret_cast<double2 *>(dcgs_scratch));
@@ -2085,7 +2140,7 @@ k_dcgs_update_bulk(ArnoldiArgs a, float2 *__restrict__ Q, int j, const float2 *_
         for (int w = 0; w < NT / 32; ++w) t += wsum[w];
         a.partial[(size_t)blk * a.pstride] = make_double2(t, 0.0);
     }
-    if (last_block_reduce(a, s, 1, st.h2 + (size_t)s * (m + 2))) {
+    if (last_block_reduce(a, s, 1, st.h2 + (size_t)s * (m + 2), nullptr)) {
         dcgs_update_finish_block(st, ds, s, m, j, rtol, max_iter, inner_rtol,
                                  reinterpret_cast<double2 *>(smem_raw));
     }

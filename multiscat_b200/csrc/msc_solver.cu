@@ -66,6 +66,16 @@ msc_status fail(msc_status st, const std::string &msg)
 // and unmaps, tens of ms); up to kPoolKeepBytes of unused memory stays
 // reserved until msc_release_cached_memory.
 constexpr int kPoolMaxDevices = 64;
+
+// A device-wide wait fails while any thread records a graph, so the two exclude
+// each other.
+std::mutex g_capture_mutex;
+cudaError_t device_sync()
+{
+    std::lock_guard<std::mutex> lock(g_capture_mutex);
+    return cudaDeviceSynchronize();
+}
+
 constexpr uint64_t kPoolKeepBytes = 32ull << 30;
 std::mutex g_pool_mutex;
 cudaMemPool_t g_pool[kPoolMaxDevices] = {};
@@ -979,10 +989,11 @@ void record_iterations_t(msc_plan *p, C2<R> *Q, C2<R> *W, C2<R> *U, cudaStream_t
                     updated = true;
                 }
             }
-            if (!updated)
-                msc::k_dcgs_update<R><<<nblk1, 256, dcgs_update_scratch_bytes(p->m), st>>>(a1, Q, j, W, p->state(), p->dstate(),
-                                                             p->m, p->desc.rtol,
-                                                             p->desc.max_iterations, inner);
+            if (!updated) {
+                auto *upd = nblk1 > 2 * 148 ? &msc::k_dcgs_update<R, 4> : &msc::k_dcgs_update<R, 8>;
+                upd<<<nblk1, 256, dcgs_update_scratch_bytes(p->m), st>>>(
+                    a1, Q, j, W, p->state(), p->dstate(), p->m, p->desc.rtol, p->desc.max_iterations, inner);
+            }
             if (tm) mark(p, 3, j, 1, st);
             continue;
         }
@@ -1006,7 +1017,7 @@ void record_iterations_t(msc_plan *p, C2<R> *Q, C2<R> *W, C2<R> *U, cudaStream_t
                            0, st);
         if (tm) mark(p, 4, j, 1, st);
     }
-    msc::k_trisolve<<<sys_blocks(p->B), 128, 0, st>>>(p->state(), p->B, p->m);
+    msc::k_trisolve<<<p->B, 32, 0, st>>>(p->state(), p->m);
     launch_update_t<R>(p, p->kcyc.p, Q, 0, p->kcyc.p, p->y.p, p->m, nullptr, nullptr, U, 1, st);
     if (tm) mark(p, 0, p->m, 0, st);
     if (p->gs || p->desc.precond_order > 0) {
@@ -1093,9 +1104,13 @@ msc_status capture(msc_plan *p, void (*rec)(msc_plan *, cudaStream_t), cudaGraph
         cudaGraphExecDestroy(*out);
         *out = nullptr;
     }
-    MSC_CUDA(cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal));
-    rec(p, p->stream);
-    cudaError_t e = cudaStreamEndCapture(p->stream, &graph);
+    cudaError_t e;
+    {
+        std::lock_guard<std::mutex> lock(g_capture_mutex);
+        MSC_CUDA(cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal));
+        rec(p, p->stream);
+        e = cudaStreamEndCapture(p->stream, &graph);
+    }
     if (e != cudaSuccess) return fail(MSC_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
     if (kernel_nodes) *kernel_nodes = count_kernel_nodes(graph);
     e = cudaGraphInstantiate(out, graph, 0);
@@ -2369,7 +2384,7 @@ msc_status msc_plan_destroy(msc_plan *plan)
     if (!plan) return MSC_OK;
     SetupTimer tm;
     cudaStreamSynchronize(plan->stream);
-    cudaDeviceSynchronize();     // nothing may still use the buffers going back to the pool
+    device_sync();               // nothing may still use the buffers going back to the pool
     delete plan;
     tm.mark("plan destroy");
     return MSC_OK;
@@ -2379,7 +2394,7 @@ msc_status msc_release_cached_memory(void)
 {
     cudaMemPool_t pool;
     MSC_CUDA(plan_pool(&pool));
-    MSC_CUDA(cudaDeviceSynchronize());
+    MSC_CUDA(device_sync());
     MSC_CUDA(cudaMemPoolTrimTo(pool, 0));
     int dev = -1;
     MSC_CUDA(cudaGetDevice(&dev));
@@ -2893,7 +2908,7 @@ msc_status msc_plan_set_adjoint(msc_plan *p, int32_t adjoint)
     const bool want = adjoint != 0;
     if (want == p->adjoint) return MSC_OK;
     // nothing of this plan may be in flight while its operator data changes
-    MSC_CUDA(cudaDeviceSynchronize());
+    MSC_CUDA(device_sync());
     const std::vector<double2> &vt = want ? p->Vt_adj_host : p->Vt_host;
     std::vector<double2> rc = p->row_c_h;
     if (want)
@@ -2903,7 +2918,7 @@ msc_status msc_plan_set_adjoint(msc_plan *p, int32_t adjoint)
     msc::k_row_cfac<<<std::min((p->R + 255) / 256, 4096), 256>>>(p->R, p->row_c.p, p->row_fn.p,
                                                                  p->row_cf.p);
     MSC_CUDA(cudaGetLastError());
-    MSC_CUDA(cudaDeviceSynchronize());    // the factors are in place before the next solve
+    MSC_CUDA(device_sync());    // the factors are in place before the next solve
     p->adjoint = want;
     if (p->sep_ok) {
         msc_status sst = upload_separable(p);
