@@ -311,6 +311,7 @@ struct msc_plan {
     // Arnoldi blocks: runs of rows of one system ("chunks", first projection)
     // and row tiles split `split` ways (update + second projection)
     int nchunks = 0;
+    bool chunk_short = false;      // one wave of blocks, a few elements per thread
     int split = 1;
     DevBuf<int> chunk_row0, chunk_nrow, chunk_sys, sys_chunk0;
     // halo-tiled coupling
@@ -351,6 +352,7 @@ struct msc_plan {
     int cycles_last = 0;
     int fallbacks_last = 0;              // systems re-solved in FP64 by the last msc_solve
     int64_t launches_cycle = 0;          // kernel nodes of the cycle graph
+    int solves = 0;                      // msc_solve calls so far
 
     ~msc_plan()
     {
@@ -990,7 +992,7 @@ void record_iterations_t(msc_plan *p, C2<R> *Q, C2<R> *W, C2<R> *U, cudaStream_t
                 }
             }
             if (!updated) {
-                auto *upd = nblk1 > 2 * 148 ? &msc::k_dcgs_update<R, 4> : &msc::k_dcgs_update<R, 8>;
+                auto *upd = p->chunk_short ? &msc::k_dcgs_update<R, 8> : &msc::k_dcgs_update<R, 4>;
                 upd<<<nblk1, 256, dcgs_update_scratch_bytes(p->m), st>>>(
                     a1, Q, j, W, p->state(), p->dstate(), p->m, p->desc.rtol, p->desc.max_iterations, inner);
             }
@@ -1045,6 +1047,17 @@ void record_cycle_iterations(msc_plan *p, cudaStream_t st)
         record_iterations_t<float>(p, p->Q32.p, p->W32.p, p->U32.p, st);
     else
         record_iterations_t<double>(p, p->Q.p, p->W.p, p->U.p, st);
+}
+
+// Kernels of one application of the preconditioner, and of one cycle with the next
+// cycle's start (what the cycle graph holds).
+int64_t cycle_launches(const msc_plan *p)
+{
+    const int k = p->desc.precond_order;
+    const int64_t pre = k <= 0 ? 1 : 2 + 3 * (int64_t)k;
+    const int64_t step = pre + 1 + (p->dcgs ? 2 : p->cgs1_inner ? 2 : 3);
+    const int64_t end = 2 + pre + (p->mixed ? 1 : p->gs || k > 0 ? 1 : 0);
+    return p->m * step + end + cycle_start_launches(false);
 }
 
 // One graph per restart cycle: its Arnoldi steps, the solution update and the next
@@ -1929,10 +1942,20 @@ msc_status finalize(msc_plan *p)
         MSC_CUDA(p->Q.alloc(vs * (m + 1)));
     }
     {
-        // Arnoldi chunks: about 4096 elements (16 per thread) per block, each
-        // block followed by one per-system reduction, but at least ~600
-        // blocks to fill the GPU; a chunk never spans two systems.
-        const int crow = std::max(1, std::min(std::max(1, 4096 / n), p->R / 600));
+        // Arnoldi chunks: up to 4096 elements (16 per thread) per block; a chunk never
+        // spans two systems.  Where that gives more blocks than one resident wave
+        // (two per SM) would take with smaller chunks, chunks stay as large as
+        // possible; below it, the smallest chunks that fit one wave: a second wave
+        // of a latency-bound pass costs as much as the first, and the last block of a
+        // system sums fewer partials.
+        const int crow_max = std::max(1, 4096 / n);
+        auto blocks_at = [&](int rows) {
+            int64_t k = 0;
+            for (int s = 0; s < p->B; ++s) k += (p->sys[s].C + rows - 1) / rows;
+            return k;
+        };
+        int crow = std::min(crow_max, std::max(1, p->R / (2 * 148)));
+        while (crow < crow_max && blocks_at(crow) > 2 * 148) ++crow;
         std::vector<int> c0, cn, cs, sc0(p->B + 1);
         for (int s = 0; s < p->B; ++s) {
             sc0[s] = (int)c0.size();
@@ -1948,6 +1971,7 @@ msc_status finalize(msc_plan *p)
         }
         sc0[p->B] = (int)c0.size();
         p->nchunks = (int)c0.size();
+        p->chunk_short = p->nchunks <= 2 * 148 && crow * n <= 2048;
         // the streamed reduction takes chunks of at most kBulkChunk elements
         // on 16-byte boundaries (n even: every chunk starts on an even element)
         const int max_rows = cn.empty() ? 0 : *std::max_element(cn.begin(), cn.end());
@@ -2043,9 +2067,6 @@ msc_status finalize(msc_plan *p)
     for (int s = 0; s < p->B; ++s) p->kcyc_host[s] = 0;
     MSC_CUDA(p->report.alloc(p->B + 1));
     MSC_CUDA(cudaStreamSynchronize(0));      // everything above is in place for the plan's stream
-    msc_status st = capture(p, record_cycle, &p->g_cycle, &p->launches_cycle);
-    if (st != MSC_OK) return st;
-    tm.mark("graph capture");
     p->finalized = true;
     return MSC_OK;
 }
@@ -2610,9 +2631,26 @@ msc_status msc_solve(msc_plan *p, double *psi_out, double *intensities_out, msc_
         live = *p->counter_host != 0;
     }
     int cycle = 0;
+    // A plan's first two solves run up to two FP64 cycles as plain launches: a one-shot
+    // call never pays for the graph (0.3 to 0.5 ms to record, build and destroy), and
+    // its kernels take longer than their launches.  Longer solves, later ones and the
+    // mixed form (three or more cycles, whose last steps are launches of systems that
+    // stopped: 2 us each, less than a plain launch takes) use one graph per cycle.
+    // Measured, ms, graph / plain: 11 x 11 x 100 2.6 / 2.3, 7 x 5 x 81 1.8 / 1.7; mixed
+    // forward and backward 41 x 41 x 200 12.4 / 13.5.
+    ++p->solves;
     for (; live && cycle < max_cycles; ++cycle) {
-        MSC_CUDA(cudaGraphLaunch(p->g_cycle, ps));
-        launches += p->launches_cycle;
+        if (!p->g_cycle && (p->mixed || p->solves > 2 || cycle >= 2)) {
+            st = capture(p, record_cycle, &p->g_cycle, &p->launches_cycle);
+            if (st != MSC_OK) return st;
+        }
+        if (p->g_cycle) {
+            MSC_CUDA(cudaGraphLaunch(p->g_cycle, ps));
+        } else {
+            record_cycle(p, ps);
+            MSC_CUDA(cudaGetLastError());
+        }
+        launches += p->g_cycle ? p->launches_cycle : cycle_launches(p);
         MSC_CUDA(cudaStreamSynchronize(ps));
         if (p->timing) accumulate_timing(p);
         live = *p->counter_host != 0;

@@ -91,3 +91,19 @@ def test_new_potentials_do_not_accumulate_device_memory():
     release_cached_memory()
     # one eigendecomposition's buffers at n = 160 are about 2 MB: 24 leaked sets would be 48 MB
     assert before - torch.cuda.mem_get_info()[0] < 16 << 20
+
+
+@pytest.mark.parametrize("options", [{}, {"precision": "mixed"}, {"gram_schmidt": "cgs2"},
+                                     {"preconditioner_order": 1}, {"gauss_seidel": True},
+                                     {"precision": "mixed", "preconditioner_order": 1, "restart": 7},
+                                     {"precision": "mixed", "inner_gram_schmidt_passes": 1}])
+def test_plain_and_graph_cycles_are_the_same_launches(options):
+    """The first two solves launch a cycle's kernels one by one, later ones as a graph:
+    same results bit for bit, same number of kernels (counted in the graph)."""
+    case = cfg0_case(nz=40)
+    plan = ScatteringPlan(case.v, case.t, [case.system()], rtol=1e-8, **options)
+    seen = [(plan.solve(), plan.launches_per_solve()) for _ in range(4)]
+    for res, launches in seen[1:]:
+        assert torch.equal(res.psi, seen[0][0].psi)
+        assert launches == seen[0][1] > 0
+    plan.close()
