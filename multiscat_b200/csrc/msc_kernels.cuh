@@ -2286,6 +2286,77 @@ k_potential_gradient(int nkx, int nky, int n, int nsys, const int *__restrict__ 
     }
 }
 
+// The same sums from shared memory: a block takes one z, stages lambda and psi of one
+// system at a time on their channel torus (absent channels zero), and each thread sums
+// KD neighbouring y offsets of one x offset.  Along a row the KD psi values a lambda
+// value meets form a window that moves by one per step: two shared-memory reads
+// (lambda a broadcast, psi free of conflicts: odd row stride, lanes in x) serve KD
+// complex FP64 MACs, so the FP64 pipe bounds it.  (The form above walks the position
+// map and L2 for every product.)  1681 x 1681 offsets and channels, n = 200: 1546 ->
+// 314 us; 122 us at the FP64 peak, the rest is latency at 12 warps per SM.
+// Grid: (chunks of dxc x offsets, z); every (D, z) is one thread's sum in a fixed order.
+template <int KD>
+__global__ void __launch_bounds__(256)
+k_gradient_planes(int nkx, int nky, int n, int nsys, const int *__restrict__ pos_map, int wx, int wy,
+                  int hx, int hy, int ndyb, int dxc, const double2 *__restrict__ psi,
+                  const double2 *__restrict__ lam, double2 *__restrict__ grad)
+{
+    extern __shared__ __align__(16) double2 gp_smem[];
+    const int ld = nky | 1, ntor = nkx * nky, z = blockIdx.y;
+    double2 *Ls = gp_smem, *Ps = gp_smem + nkx * ld;
+    const int yb = threadIdx.x / dxc, u = blockIdx.x * dxc + (threadIdx.x - yb * dxc);
+    const bool work = yb < ndyb && u < wx;
+    const int dx = ((u - hx) % nkx + nkx) % nkx, dy0 = ((yb * KD - hy) % nky + nky) % nky;
+    const int i0 = (nky - dy0) % nky;             // psi row position that lambda's first meets at dy0
+    double2 acc[KD];
+#pragma unroll
+    for (int k = 0; k < KD; ++k) acc[k] = make_double2(0.0, 0.0);
+    for (int s = 0; s < nsys; ++s) {
+        const int *map = pos_map + (size_t)s * ntor;
+        if (s > 0) __syncthreads();
+        for (int i = threadIdx.x; i < ntor; i += blockDim.x) {
+            const int r = __ldg(map + i), x = i / nky, y = i - x * nky;
+            const double2 zero = make_double2(0.0, 0.0);
+            Ls[x * ld + y] = r >= 0 ? lam[(size_t)r * n + z] : zero;
+            Ps[x * ld + y] = r >= 0 ? psi[(size_t)r * n + z] : zero;
+        }
+        __syncthreads();
+        if (!work) continue;
+        for (int gx = 0; gx < nkx; ++gx) {
+            const double2 *lrow = Ls + gx * ld;
+            const double2 *prow = Ps + (gx - dx + (gx < dx ? nkx : 0)) * ld;
+            // window slot (step - k) mod KD holds psi(step - dy0 - k)
+            double2 w[KD];
+#pragma unroll
+            for (int k = 1; k < KD; ++k) w[KD - k] = prow[((i0 - k) % nky + nky) % nky];
+            int cur = i0;
+            for (int g0 = 0; g0 < nky; g0 += KD) {
+#pragma unroll
+                for (int r = 0; r < KD; ++r) {
+                    const double2 l = g0 + r < nky ? lrow[g0 + r] : make_double2(0.0, 0.0);
+                    w[r] = prow[cur];
+                    cur = cur + 1 == nky ? 0 : cur + 1;
+#pragma unroll
+                    for (int k = 0; k < KD; ++k) {
+                        const double2 q = w[(r - k + KD) % KD];
+                        acc[k].x = fma(l.x, q.x, fma(l.y, q.y, acc[k].x));
+                        acc[k].y = fma(l.x, q.y, fma(-l.y, q.x, acc[k].y));
+                    }
+                }
+            }
+        }
+    }
+    if (!work) return;
+#pragma unroll
+    for (int k = 0; k < KD; ++k) {
+        if (yb * KD + k >= wy) break;
+        const int dy = (dy0 + k) % nky;
+        grad[((size_t)dx * nky + dy) * n + z] =
+            dx == 0 && dy == 0 ? make_double2(-2.0 * acc[k].x, 0.0)
+                               : make_double2(-2.0 * acc[k].x, 2.0 * acc[k].y);
+    }
+}
+
 // Plan set-up on the device, one thread per channel row:
 //   fn[row]  = sum_k E[n-1,k]^2 / (pkd_row + lam_k)   (Sherman-Morrison factor
 //              of the block inverse, multiscat_gmres.f90:226-273)

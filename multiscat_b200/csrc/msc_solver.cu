@@ -1194,6 +1194,10 @@ msc_status set_kernel_attributes()
                                   (int)msc::dcgs_bulk_smem()));
     MSC_CUDA(cudaFuncSetAttribute(msc::k_dcgs_update_bulk, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)msc::dcgs_bulk_smem()));
+    MSC_CUDA(cudaFuncSetAttribute(msc::k_gradient_planes<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+    MSC_CUDA(cudaFuncSetAttribute(msc::k_gradient_planes<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+    MSC_CUDA(cudaFuncSetAttribute(msc::k_gradient_planes<7>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+    MSC_CUDA(cudaFuncSetAttribute(msc::k_gradient_planes<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
     done[dev] = true;
     return MSC_OK;
 }
@@ -3032,7 +3036,38 @@ msc_status msc_potential_gradient(msc_plan *p, const double *psi, const double *
         hy = half_y;
     }
     cudaStream_t us = reinterpret_cast<cudaStream_t>(stream);
-    MSC_CUDA(cudaMemsetAsync(grad, 0, (size_t)ntor * n * sizeof(double2), us));
+    if (wx < nkx || wy < nky)
+        MSC_CUDA(cudaMemsetAsync(grad, 0, (size_t)ntor * n * sizeof(double2), us));
+    // Both planes of one z in shared memory (up to 7200 torus positions), else the form
+    // that reads them from L2.  KD: the offsets per thread that leave the least padding;
+    // x offsets are cut until there are about four blocks per SM.
+    const size_t plane_bytes = (size_t)2 * nkx * (nky | 1) * sizeof(double2);
+    if (plane_bytes <= 226 * 1024) {
+        int kd = 8, best = 1 << 30;
+        for (int k = 5; k <= 8; ++k) {
+            const int cost = (wy + k - 1) / k * k * ((nky + k - 1) / k * k);
+            if (cost <= best) {
+                best = cost;
+                kd = k;
+            }
+        }
+        const int ndyb = (wy + kd - 1) / kd;
+        const int dx_max = std::max(1, 256 / ndyb);
+        if (ndyb <= 256) {
+            const int want = std::max((wx + dx_max - 1) / dx_max, std::min(wx, (4 * 148 + n - 1) / n));
+            const int dxc = (wx + want - 1) / want;
+            const dim3 g((wx + dxc - 1) / dxc, n);
+            const int nt = (dxc * ndyb + 31) / 32 * 32;
+            auto *kern = kd == 5 ? &msc::k_gradient_planes<5> : kd == 6 ? &msc::k_gradient_planes<6>
+                         : kd == 7 ? &msc::k_gradient_planes<7> : &msc::k_gradient_planes<8>;
+            kern<<<g, nt, plane_bytes, us>>>(nkx, nky, n, p->B, p->pos_map.p, wx, wy, hx, hy, ndyb, dxc,
+                                             reinterpret_cast<const double2 *>(psi),
+                                             reinterpret_cast<const double2 *>(lambda),
+                                             reinterpret_cast<double2 *>(grad));
+            MSC_CUDA(cudaGetLastError());
+            return MSC_OK;
+        }
+    }
     const int per_block = 8 * msc::kGradPerWarp;
     dim3 grid((wx * wy + per_block - 1) / per_block, (n + 31) / 32);
     msc::k_potential_gradient<<<grid, 256, 0, us>>>(
