@@ -47,7 +47,9 @@ inline int tridiagonal_qr_rotations(int n, std::vector<double> &d, std::vector<d
         const double shift = d[hi] - eh * eh / (half + std::copysign(std::hypot(half, eh), half));
         double x = d[lo] - shift, y = e[lo];
         for (int k = lo; k < hi; ++k) {
-            const double r = std::hypot(x, y);
+            // sqrt of the sum where neither square leaves the range, else hypot
+            const double r2 = x * x + y * y;
+            const double r = r2 > 1e-280 && r2 < 1e280 ? std::sqrt(r2) : std::hypot(x, y);
             const double c = (r == 0.0) ? 1.0 : x / r;
             const double s = (r == 0.0) ? 0.0 : y / r;
             if (k > lo) e[k - 1] = r;

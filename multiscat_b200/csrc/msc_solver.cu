@@ -2160,8 +2160,10 @@ msc_status ensure_gs_levels(msc_plan *p)
 msc_status device_symmetric_eigh(int n, const double *H, double *w, double *E)
 {
     namespace eg = msc::eig;
-    DevBuf<double> A, R, d, e, Zt, Ed, rc, rs;
-    DevBuf<int> applied, rk, dest;
+    DevBuf<double> A, R, d, e, Zt, Ed;
+    DevBuf<int> applied, dest;
+    DevBuf<int4> groups;
+    DevBuf<double2> tab;
     std::vector<double> Hh(H, H + (size_t)n * n);
     MSC_CUDA(upload(A, Hh));
     MSC_CUDA(R.alloc((size_t)n * n));
@@ -2170,10 +2172,44 @@ msc_status device_symmetric_eigh(int n, const double *H, double *w, double *E)
     MSC_CUDA(applied.alloc(n));
     MSC_CUDA(cudaMemsetAsync(R.p, 0, (size_t)n * n * sizeof(double), 0));
     MSC_CUDA(cudaMemsetAsync(e.p, 0, (size_t)n * sizeof(double), 0));
-    const size_t tri_smem = n <= eg::kTriSmemMaxN ? (size_t)n * n * sizeof(double) : 0;
-    MSC_CUDA(cudaFuncSetAttribute(eg::k_tridiagonalize, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)((size_t)eg::kTriSmemMaxN * eg::kTriSmemMaxN * sizeof(double))));
-    eg::k_tridiagonalize<<<1, eg::kTriThreads, tri_smem>>>(n, A.p, R.p, d.p, e.p, applied.p);
+    // one CTA while the matrix fits its shared memory; a cluster of 8, then of 16
+    // (where the device grants that size) while it fits theirs; else one CTA from L2
+    int cl = 0;
+    constexpr size_t kRoom = 226 * 1024;
+    if (n > eg::kTriSmemMaxN) {
+        MSC_CUDA(cudaFuncSetAttribute(eg::k_tridiagonalize_cluster,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRoom));
+        MSC_CUDA(cudaFuncSetAttribute(eg::k_tridiagonalize_cluster,
+                                      cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        for (int c : {8, 16}) {
+            if (eg::tri_cluster_smem(n, c) > kRoom) continue;
+            cudaLaunchConfig_t lc{};
+            lc.gridDim = dim3(c);
+            lc.blockDim = dim3(eg::kTriThreads);
+            lc.dynamicSmemBytes = eg::tri_cluster_smem(n, c);
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = c;
+            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+            lc.attrs = at;
+            lc.numAttrs = 1;
+            int nclusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&nclusters, eg::k_tridiagonalize_cluster, &lc) != cudaSuccess ||
+                nclusters < 1) {
+                (void)cudaGetLastError();
+                continue;
+            }
+            cl = c;
+            MSC_CUDA(cudaLaunchKernelEx(&lc, eg::k_tridiagonalize_cluster, n, (const double *)A.p, R.p, d.p, e.p,
+                                        applied.p));
+            break;
+        }
+    }
+    if (cl == 0) {
+        MSC_CUDA(cudaFuncSetAttribute(eg::k_tridiagonalize, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)eg::tri_smem(eg::kTriSmemMaxN)));
+        eg::k_tridiagonalize<<<1, eg::kTriThreads, eg::tri_smem(n)>>>(n, A.p, R.p, d.p, e.p, applied.p);
+    }
     MSC_CUDA(cudaGetLastError());
     std::vector<double> dh(n), eh(n);
     MSC_CUDA(cudaMemcpy(dh.data(), d.p, n * sizeof(double), cudaMemcpyDeviceToHost));
@@ -2186,26 +2222,52 @@ msc_status device_symmetric_eigh(int n, const double *H, double *w, double *E)
     rsh.reserve((size_t)n * n);
     if (msc::tridiagonal_qr_rotations(n, dh, eh, rkh, rch, rsh) != 0)
         return fail(MSC_ERR_EIGEN, "eigensolver did not converge");
-    const int nrot = (int)rkh.size();
-    if (nrot > 0) {
-        MSC_CUDA(upload(rk, rkh));
-        MSC_CUDA(upload(rc, rch));
-        MSC_CUDA(upload(rs, rsh));
+    // sweeps of rising k in groups of four, each group's coefficients per step (sweep j
+    // two columns behind sweep j - 1), identity where a sweep does not reach
+    {
+        std::vector<int4> gh;
+        std::vector<double2> th;
+        const size_t nrot = rkh.size();
+        th.reserve(4 * (nrot / 3 + 64));
+        for (size_t i = 0; i < nrot;) {
+            size_t at[5];
+            int ns = 0, lo = n, hi = 0;
+            size_t q = i;
+            while (ns < 4 && q < nrot) {
+                at[ns++] = q;
+                const size_t first = q++;
+                while (q < nrot && rkh[q] == rkh[q - 1] + 1) ++q;
+                lo = std::min(lo, rkh[first]);
+                hi = std::max(hi, rkh[q - 1] + 1);
+            }
+            at[ns] = q;
+            const int L = hi - lo, steps = L + 6;
+            const size_t base = th.size();
+            gh.push_back(make_int4(lo, hi, (int)(base / 4), 0));
+            th.resize(base + (size_t)steps * 4, make_double2(1.0, 0.0));
+            for (int j = 0; j < ns; ++j)
+                for (size_t r = at[j]; r < at[j + 1]; ++r)
+                    th[base + (size_t)(rkh[r] - lo + 2 * j) * 4 + j] = make_double2(rch[r], rsh[r]);
+            i = q;
+        }
+        if (!gh.empty()) {
+            MSC_CUDA(upload(groups, gh));
+            MSC_CUDA(upload(tab, th));
+        }
+        MSC_CUDA(Zt.alloc((size_t)n * n));
+        // rows of Z per CTA: as many as fit shared memory (32 or 16)
+        const int nsteps = (int)(th.size() / 4), ng = (int)gh.size();
+        auto rotate = [&](auto kern, int rb, size_t sm) -> cudaError_t {
+            cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRoom);
+            if (ce == cudaSuccess) kern<<<(n + rb - 1) / rb, 32, sm>>>(n, ng, nsteps, groups.p, tab.p, Zt.p);
+            return ce;
+        };
+        if (eg::rotations_smem<32>(n) <= kRoom)
+            MSC_CUDA(rotate(&eg::k_apply_rotations<32>, 32, eg::rotations_smem<32>(n)));
+        else
+            MSC_CUDA(rotate(&eg::k_apply_rotations<16>, 16, eg::rotations_smem<16>(n)));
+        MSC_CUDA(cudaGetLastError());
     }
-    MSC_CUDA(Zt.alloc((size_t)n * n));
-    // rows of Z per CTA: as many as fit 200 KB of shared memory (32 or 16)
-    if ((size_t)n * 32 * sizeof(double) <= 200 * 1024) {
-        const size_t sm = (size_t)n * 32 * sizeof(double);
-        MSC_CUDA(cudaFuncSetAttribute(eg::k_apply_rotations<32>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        eg::k_apply_rotations<32><<<(n + 31) / 32, 32, sm>>>(n, nrot, rk.p, rc.p, rs.p, Zt.p);
-    } else {
-        const size_t sm = (size_t)n * 16 * sizeof(double);
-        MSC_CUDA(cudaFuncSetAttribute(eg::k_apply_rotations<16>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        eg::k_apply_rotations<16><<<(n + 15) / 16, 16, sm>>>(n, nrot, rk.p, rc.p, rs.p, Zt.p);
-    }
-    MSC_CUDA(cudaGetLastError());
     // ascending order: column j of Q_H Z goes to column dest[j]
     std::vector<int> order(n), desth(n);
     std::iota(order.begin(), order.end(), 0);
@@ -2216,17 +2278,13 @@ msc_status device_symmetric_eigh(int n, const double *H, double *w, double *E)
     }
     MSC_CUDA(upload(dest, desth));
     MSC_CUDA(Ed.alloc((size_t)n * n));
-    if ((size_t)n * 32 * sizeof(double) <= 200 * 1024) {
-        const size_t sm = (size_t)n * 32 * sizeof(double);
-        MSC_CUDA(cudaFuncSetAttribute(eg::k_back_transform<32>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        eg::k_back_transform<32><<<(n + 31) / 32, 256, sm>>>(n, R.p, applied.p, Zt.p, dest.p, Ed.p);
-    } else {
-        const size_t sm = (size_t)n * 16 * sizeof(double);
-        MSC_CUDA(cudaFuncSetAttribute(eg::k_back_transform<16>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        eg::k_back_transform<16><<<(n + 15) / 16, 256, sm>>>(n, R.p, applied.p, Zt.p, dest.p, Ed.p);
-    }
+    auto back = [&](auto kern, int cb) {
+        kern<<<(n + 4 * cb - 1) / (4 * cb), 128>>>(n, R.p, applied.p, Zt.p, dest.p, Ed.p);
+    };
+    if (n <= 128) back(&eg::k_back_transform<4, 2>, 2);
+    else if (n <= 256) back(&eg::k_back_transform<8, 2>, 2);
+    else if (n <= 512) back(&eg::k_back_transform<16, 2>, 2);
+    else back(&eg::k_back_transform<32, 1>, 1);
     MSC_CUDA(cudaGetLastError());
     MSC_CUDA(cudaMemcpy(E, Ed.p, (size_t)n * n * sizeof(double), cudaMemcpyDeviceToHost));
     return MSC_OK;
