@@ -509,190 +509,6 @@ k_gs_sweep(int nsys, const int *__restrict__ gate, int n, int K,
 }
 
 // ---------------------------------------------------------------------------
-// Channel coupling with shared-memory halo tiles (the hot form of k_coupling).
-//
-// A block owns an 8 x BX patch of torus positions of ONE system and ZC
-// consecutive z.  It stages the patch plus a halo of HX (x) and HY (y)
-// positions -- the reach of the coupling taps -- for its z range in shared
-// memory (absent channels, i.e. positions outside a truncated channel set,
-// read as zero; positions wrap around the torus exactly as the reference's
-// modulo(G_j - G_i, n) does).  Each thread keeps one column of YS + 2 HY halo
-// values in registers and produces YS outputs along y for one (x, z):
-// for every tap (sdx, sdy) in the window it issues YS complex FMAs from
-// registers, so a halo value loaded once serves up to 2 HY + 1 taps.
-//   out[r] = in0[r] + sgn * sum_t V_t(z) src[pos(r) - delta_t](z)
-// ---------------------------------------------------------------------------
-struct CouplingTiles {
-    const int *work;          // [nwork][3]: system, x0, y0
-    const int *pos_row;       // [B][nkx * nky]: row of each torus position, -1 if absent
-    const int *tap_window;    // [(2 HX + 1) * (2 HY + 1)]: tap index per signed offset, -1 if none
-    int nwork, nkx, nky, hx;  // hx = HX (runtime); HY is the template parameter
-    int ntaps;                // K
-};
-
-// MASK 1 / 2: only the source channels with a smaller / larger row index
-// than the output's (V^lower / V^upper of the block Gauss-Seidel splitting,
-// as k_coupling_masked); 0: the full coupling.
-template <int HY, int BX, int ZC, int YS, typename R, int MASK = 0>
-__global__ void __launch_bounds__(BX * ZC * (8 / YS))
-k_coupling_halo(CouplingTiles ct, const int *__restrict__ gate, int n,
-                const typename CT<R>::t *__restrict__ Vt, const typename CT<R>::t *__restrict__ src,
-                const typename CT<R>::t *__restrict__ in0, R sgn, typename CT<R>::t *__restrict__ out)
-{
-    // YS outputs along y per thread; 8 / YS threads share one (x, z) column.
-    using C2 = typename CT<R>::t;
-    constexpr int BY = 8;
-    constexpr int HYW = BY + 2 * HY;
-    constexpr int WY = 2 * HY + 1;
-    constexpr int NT = BX * ZC * (BY / YS);
-    constexpr int CW = YS + 2 * HY;              // halo values one thread keeps per column
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int HX = ct.hx;
-    const int HXW = BX + 2 * HX;
-    const int nwin = (2 * HX + 1) * WY;
-    C2 *halo = reinterpret_cast<C2 *>(smem_raw);                              // [HXW][HYW][ZC]
-    C2 *vw = halo + (size_t)HXW * HYW * ZC;                                   // [window cell][ZC]
-    int *rows = reinterpret_cast<int *>(vw + (size_t)nwin * ZC);              // [HXW][HYW]
-    // Threads whose y segment (YS positions) of their patch column holds no
-    // channel skip the tap loop (truncated channel sets leave many near the
-    // edge of the channel disk); the test reads the staged rows table.
-
-    const int w = blockIdx.x;
-    const int s = ct.work[3 * w];
-    if (gate && gate[s] == 0) return;
-    const int x0 = ct.work[3 * w + 1], y0 = ct.work[3 * w + 2];
-    const int z0 = blockIdx.y * ZC;
-    const int nkx = ct.nkx, nky = ct.nky;
-    const int *pr = ct.pos_row + (size_t)s * nkx * nky;
-    // tap values of this z range, one row per window cell (zero where no tap)
-    for (int i = threadIdx.x; i < nwin * ZC; i += NT) {
-        const int cell = i / ZC, z = z0 + (i % ZC);
-        const int t = ct.tap_window[cell];
-        vw[i] = (t >= 0 && z < n) ? Vt[(size_t)t * n + z] : mk2<R>(0, 0);
-    }
-    // source row of every halo position (absent channels: -1)
-    const int npos = HXW * HYW;
-    for (int pidx = threadIdx.x; pidx < npos; pidx += NT) {
-        const int hy = pidx % HYW, hx = pidx / HYW;
-        int gx = (x0 + hx - HX) % nkx;
-        if (gx < 0) gx += nkx;
-        int gy = (y0 + hy - HY) % nky;
-        if (gy < 0) gy += nky;
-        rows[pidx] = pr[gx * nky + gy];
-    }
-    __syncthreads();
-    constexpr int kU = 8;
-    const int total = npos * ZC;
-    if (std::is_same<R, float>::value && (n % 2) == 0) {
-        // FP32, n even: two consecutive z per 16-byte load (z0 and ZC are even)
-        const int total2 = total / 2;
-        float4 *halo4 = reinterpret_cast<float4 *>(halo);
-        for (int base = threadIdx.x; base < total2; base += NT * kU) {
-            float4 v[kU];
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int idx = base + u * NT;
-                v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (idx < total2) {
-                    const int row = rows[(2 * idx) / ZC];
-                    const int z = z0 + ((2 * idx) % ZC);
-                    if (row >= 0 && z < n)    // z < n implies z + 1 < n (both even)
-                        v[u] = *reinterpret_cast<const float4 *>(src + (size_t)row * n + z);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int idx = base + u * NT;
-                if (idx < total2) halo4[idx] = v[u];
-            }
-        }
-    } else {
-        for (int base = threadIdx.x; base < total; base += NT * kU) {
-            C2 v[kU];
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int idx = base + u * NT;
-                v[u] = mk2<R>(0, 0);
-                if (idx < total) {
-                    const int row = rows[idx / ZC];
-                    const int z = z0 + (idx % ZC);
-                    if (row >= 0 && z < n) v[u] = src[(size_t)row * n + z];
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int idx = base + u * NT;
-                if (idx < total) halo[idx] = v[u];
-            }
-        }
-    }
-    __syncthreads();
-
-    const int zl = threadIdx.x % ZC;
-    const int tx = (threadIdx.x / ZC) % BX;
-    const int ysub = threadIdx.x / (ZC * BX);      // which YS-slice of the 8 y outputs
-    const int z = z0 + zl;
-    bool any = false;
-#pragma unroll
-    for (int y = ysub * YS; y < (ysub + 1) * YS; ++y)
-        any |= (y0 + y < nky) && rows[(tx + HX) * HYW + y + HY] >= 0;
-    if (x0 + tx >= nkx || z >= n || !any) return;
-    R ar[YS], ai[YS];
-#pragma unroll
-    for (int y = 0; y < YS; ++y) {
-        ar[y] = 0;
-        ai[y] = 0;
-    }
-    int orow[MASK ? YS : 1];
-    if (MASK) {
-#pragma unroll
-        for (int y = 0; y < YS; ++y) orow[y] = rows[(tx + HX) * HYW + ysub * YS + y + HY];
-    }
-    for (int sdx = -HX; sdx <= HX; ++sdx) {
-        const int hx = tx - sdx + HX;
-        const C2 *colp = halo + ((size_t)hx * HYW + ysub * YS) * ZC + zl;
-        C2 col[CW];
-#pragma unroll
-        for (int i = 0; i < CW; ++i) col[i] = colp[(size_t)i * ZC];
-        int crow[MASK ? CW : 1];
-        if (MASK) {
-#pragma unroll
-            for (int i = 0; i < CW; ++i) crow[i] = rows[hx * HYW + ysub * YS + i];
-        }
-        const C2 *vrow = vw + (size_t)(sdx + HX) * WY * ZC + zl;
-#pragma unroll
-        for (int sdy = -HY; sdy <= HY; ++sdy) {
-            const C2 v = vrow[(sdy + HY) * ZC];
-#pragma unroll
-            for (int y = 0; y < YS; ++y) {
-                C2 q = col[y - sdy + HY];
-                if (MASK) {
-                    const int sr = crow[MASK ? y - sdy + HY : 0], orr = orow[MASK ? y : 0];
-                    const bool keep = MASK == 1 ? sr < orr : sr > orr;
-                    if (!keep) q = mk2<R>(0, 0);
-                }
-                ar[y] = fma(v.x, q.x, fma(-v.y, q.y, ar[y]));
-                ai[y] = fma(v.x, q.y, fma(v.y, q.x, ai[y]));
-            }
-        }
-    }
-    // output rows from the staged rows table; the in0 loads of all YS
-    // outputs go out before the stores
-    int rowv[YS];
-    C2 base[YS];
-#pragma unroll
-    for (int y = 0; y < YS; ++y)
-        rowv[y] = (y0 + ysub * YS + y < nky) ? rows[(tx + HX) * HYW + ysub * YS + y + HY] : -1;
-#pragma unroll
-    for (int y = 0; y < YS; ++y)
-        base[y] = (in0 && rowv[y] >= 0) ? in0[(size_t)rowv[y] * n + z] : mk2<R>(0, 0);
-#pragma unroll
-    for (int y = 0; y < YS; ++y)
-        if (rowv[y] >= 0)
-            out[(size_t)rowv[y] * n + z] = mk2<R>(base[y].x + sgn * ar[y], base[y].y + sgn * ai[y]);
-}
-
-// ---------------------------------------------------------------------------
 // Arnoldi reductions.  partial[tile][i] = sum conj(Q_i) W over the tile for
 // i < nvec; slot nvec holds ||W||^2 when with_norm.  One warp per vector;
 // FP64 accumulation for both precisions.

@@ -36,6 +36,7 @@
 #include "msc_common.cuh"
 #include "msc_dmma.cuh"
 #include "msc_eigh.hpp"
+#include "msc_halo.cuh"
 #include "msc_eigh_gpu.cuh"
 #include "msc_kernels.cuh"
 #include "msc_tc.cuh"
@@ -317,7 +318,7 @@ struct msc_plan {
     // halo-tiled coupling
     bool use_halo = false;             // halo tables built (taps reach <= 8)
     int halo32 = 0, halo64 = 0;    // autotuned coupling kind per precision (0 nbr, 1/2 halo)
-    int halo_hx = 0, halo_hy = 0, nwork = 0;
+    int halo_hx = 0, halo_hy = 0, halo_bx = 0, halo_by = 0, halo_seg = 1, nwork = 0;
     // separable coupling (coupling kinds 3 to 5): p, q, kappa per z when every tap
     // window factorises (see k_coupling_box); host copies for the adjoint
     bool sep_ok = false;
@@ -335,7 +336,8 @@ struct msc_plan {
     // autotuning record: microseconds per candidate
     std::vector<std::pair<std::string, float>> tune_log;
     std::string tune_report;
-    DevBuf<int> work, tap_window;
+    DevBuf<int4> work;
+    DevBuf<int> tap_window;
     DevBuf<int2> taps_d;                      // [K] tap offsets (dx, dy)
     DevBuf<int> sys_counter;       // per-system arrival counters of the fused Arnoldi kernels
     cudaStream_t stream = nullptr;
@@ -592,39 +594,68 @@ void launch_residual_diag(msc_plan *p, const int *gate, const double2 *x, double
     (void)msc::dm::dispatch(false, msc::dm::choose(p->R, p->n), q, st, true);
 }
 
-constexpr int kHaloBX = 8;
-template <typename R> constexpr int halo_zc() { return std::is_same<R, float>::value ? 32 : 16; }
-
-size_t halo_smem(int hx, int hy, int zc, size_t elem)
+// The halo kernel instance of (window reach, outputs per thread, precision, mask) as a
+// call of f(kernel).
+template <int HY, typename R, int MASK, typename F>
+auto halo_instance_ys(int ys, F f)
 {
-    return (size_t)(kHaloBX + 2 * hx) * (8 + 2 * hy) * zc * elem +
-           (size_t)(2 * hx + 1) * (2 * hy + 1) * zc * elem +
-           (size_t)(kHaloBX + 2 * hx) * (8 + 2 * hy) * sizeof(int);
+    if constexpr (MASK != 0) {
+        return ys == 3 ? f(&msc::k_coupling_halo<HY, 3, R, MASK>) : f(&msc::k_coupling_halo<HY, 4, R, MASK>);
+    } else {
+        switch (ys) {
+        case 3: return f(&msc::k_coupling_halo<HY, 3, R, 0>);
+        case 4: return f(&msc::k_coupling_halo<HY, 4, R, 0>);
+        case 5: return f(&msc::k_coupling_halo<HY, 5, R, 0>);
+        case 6: return f(&msc::k_coupling_halo<HY, 6, R, 0>);
+        case 7: return f(&msc::k_coupling_halo<HY, 7, R, 0>);
+        default: return f(&msc::k_coupling_halo<HY, 8, R, 0>);
+        }
+    }
 }
 
-template <int HY, int YS, typename R, int MASK = 0>
-void launch_halo(msc_plan *p, const int *gate, const C2<R> *src, const C2<R> *in0, R sgn,
+template <typename R, int MASK, typename F>
+auto halo_instance(int hy, int ys, F f)
+{
+    switch (hy) {
+    case 1: return halo_instance_ys<1, R, MASK>(ys, f);
+    case 2: return halo_instance_ys<2, R, MASK>(ys, f);
+    case 4: return halo_instance_ys<4, R, MASK>(ys, f);
+    default: return halo_instance_ys<8, R, MASK>(ys, f);
+    }
+}
+
+// Shared memory of every instance: set once per device (a block never asks for more
+// than the largest halo, 8 + 16 by 16 + 16 positions with 17 x 17 taps).
+template <typename R, int MASK>
+cudaError_t halo_attributes()
+{
+    for (int hy = 1; hy <= 8; hy *= 2)
+        for (int ys = 3; ys <= (MASK ? 4 : 8); ++ys) {
+            const size_t smem = msc::halo_smem(8, hy, msc::kHaloMax, 2 * msc::kHaloMax,
+                                               msc::halo_zc<R>(), sizeof(C2<R>));
+            const cudaError_t e = halo_instance<R, MASK>(hy, ys, [&](auto kernel) {
+                return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            });
+            if (e != cudaSuccess) return e;
+        }
+    return cudaSuccess;
+}
+
+// kind 1: a thread takes half or all of a patch column (5 to 8 outputs, 3 or 4 of low
+// patches), kind 2 and the masked forms: half of that.
+template <typename R, int MASK = 0>
+void launch_halo(msc_plan *p, int kind, const int *gate, const C2<R> *src, const C2<R> *in0, R sgn,
                  C2<R> *out, cudaStream_t st)
 {
-    constexpr int ZC = halo_zc<R>();
-    msc::CouplingTiles ct{p->work.p, p->pos_map.p, p->tap_window.p, p->nwork, p->nkx, p->nky,
-                          p->halo_hx, p->K};
-    dim3 grid(p->nwork, (p->n + ZC - 1) / ZC);
-    msc::k_coupling_halo<HY, kHaloBX, ZC, YS, R, MASK>
-        <<<grid, kHaloBX * ZC * (8 / YS), halo_smem(p->halo_hx, HY, ZC, sizeof(C2<R>)), st>>>(
+    constexpr int ZC = msc::halo_zc<R>();
+    const int ns = kind * p->halo_seg, ys = msc::halo_ys(p->halo_by, ns);
+    const msc::CouplingTiles ct{p->work.p, p->pos_map.p, p->tap_window.p, p->nwork, p->nkx, p->nky,
+                                p->halo_hx, p->halo_bx, p->halo_by, ns};
+    const size_t smem = msc::halo_smem(p->halo_hx, p->halo_hy, p->halo_bx, ns * ys, ZC, sizeof(C2<R>));
+    halo_instance<R, MASK>(p->halo_hy, ys, [&](auto kernel) {
+        kernel<<<dim3(p->nwork, (p->n + ZC - 1) / ZC), p->halo_bx * ZC * ns, smem, st>>>(
             ct, gate, p->n, OpData<R>::Vt(p), src, in0, sgn, out);
-}
-
-template <int YS, typename R, int MASK = 0>
-void launch_halo_ys(msc_plan *p, const int *gate, const C2<R> *src, const C2<R> *in0, R sgn,
-                    C2<R> *out, cudaStream_t st)
-{
-    switch (p->halo_hy) {
-    case 1: launch_halo<1, YS, R, MASK>(p, gate, src, in0, sgn, out, st); return;
-    case 2: launch_halo<2, YS, R, MASK>(p, gate, src, in0, sgn, out, st); return;
-    case 4: launch_halo<4, YS, R, MASK>(p, gate, src, in0, sgn, out, st); return;
-    default: launch_halo<8, YS, R, MASK>(p, gate, src, in0, sgn, out, st); return;
-    }
+    });
 }
 
 // The box kernel instance of (window reach, precision, kind) as a call of f(shape, kernel).
@@ -728,12 +759,12 @@ template <typename R>
 void launch_coupling_t(msc_plan *p, const int *gate, const C2<R> *src, const C2<R> *in0, R sgn,
                        C2<R> *out, cudaStream_t st)
 {
-    // coupling kind per precision: 0 neighbour table, 1 halo (8 y/thread), 2 halo (4 y/thread),
+    // coupling kind per precision: 0 neighbour table, 1 / 2 halo tiles with one / two
+    // threads per patch column,
     // 3 to 5 separable over channel boxes (two 1-D passes; only when the tap windows
     // factorise), with the most, half and a quarter of the z per block
     const int kind = p->use_halo ? (std::is_same<R, float>::value ? p->halo32 : p->halo64) : 0;
-    if (kind == 1) { launch_halo_ys<8, R>(p, gate, src, in0, sgn, out, st); return; }
-    if (kind == 2) { launch_halo_ys<4, R>(p, gate, src, in0, sgn, out, st); return; }
+    if (kind == 1 || kind == 2) { launch_halo<R>(p, kind, gate, src, in0, sgn, out, st); return; }
     if (kind >= 3 && p->sep_ok) {
         launch_boxes<R>(p, kind, gate, src, in0, sgn, out, st);
         return;
@@ -759,8 +790,8 @@ void launch_coupling_masked_t(msc_plan *p, const int *gate, const C2<R> *src, co
                               R sgn, int mask, C2<R> *out, cudaStream_t st)
 {
     if (p->use_halo) {
-        if (mask == 1) launch_halo_ys<4, R, 1>(p, gate, src, in0, sgn, out, st);
-        else launch_halo_ys<4, R, 2>(p, gate, src, in0, sgn, out, st);
+        if (mask == 1) launch_halo<R, 1>(p, 2, gate, src, in0, sgn, out, st);
+        else launch_halo<R, 2>(p, 2, gate, src, in0, sgn, out, st);
         return;
     }
     dim3 grid(p->ntiles, (p->n + 31) / 32);
@@ -1151,35 +1182,12 @@ msc_status set_kernel_attributes()
                                   (int)smem_block_inverse_t<float>(msc::kMaxNz)));
     MSC_CUDA(cudaFuncSetAttribute(msc::k_coupling<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)smem_coupling(msc::kMaxTaps)));
-#define MSC_HALO_ATTR(HY, R)                                                                     \
-    MSC_CUDA(cudaFuncSetAttribute(msc::k_coupling_halo<HY, kHaloBX, halo_zc<R>(), 8, R>,        \
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,                   \
-                                  (int)std::min<size_t>(halo_smem(8, HY, halo_zc<R>(), sizeof(C2<R>)), 232448))); \
-    MSC_CUDA(cudaFuncSetAttribute(msc::k_coupling_halo<HY, kHaloBX, halo_zc<R>(), 4, R>,        \
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,                   \
-                                  (int)std::min<size_t>(halo_smem(8, HY, halo_zc<R>(), sizeof(C2<R>)), 232448)));;
-#define MSC_HALO_MASK_ATTR(HY, R, M)                                                              \
-    MSC_CUDA(cudaFuncSetAttribute(msc::k_coupling_halo<HY, kHaloBX, halo_zc<R>(), 4, R, M>,       \
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,                   \
-                                  (int)std::min<size_t>(halo_smem(8, HY, halo_zc<R>(), sizeof(C2<R>)), 232448)));
-    MSC_HALO_MASK_ATTR(1, float, 1) MSC_HALO_MASK_ATTR(2, float, 1)
-    MSC_HALO_MASK_ATTR(4, float, 1) MSC_HALO_MASK_ATTR(8, float, 1)
-    MSC_HALO_MASK_ATTR(1, float, 2) MSC_HALO_MASK_ATTR(2, float, 2)
-    MSC_HALO_MASK_ATTR(4, float, 2) MSC_HALO_MASK_ATTR(8, float, 2)
-    MSC_HALO_MASK_ATTR(1, double, 1) MSC_HALO_MASK_ATTR(2, double, 1)
-    MSC_HALO_MASK_ATTR(4, double, 1) MSC_HALO_MASK_ATTR(8, double, 1)
-    MSC_HALO_MASK_ATTR(1, double, 2) MSC_HALO_MASK_ATTR(2, double, 2)
-    MSC_HALO_MASK_ATTR(4, double, 2) MSC_HALO_MASK_ATTR(8, double, 2)
-#undef MSC_HALO_MASK_ATTR
-    MSC_HALO_ATTR(1, float)
-    MSC_HALO_ATTR(2, float)
-    MSC_HALO_ATTR(4, float)
-    MSC_HALO_ATTR(8, float)
-    MSC_HALO_ATTR(1, double)
-    MSC_HALO_ATTR(2, double)
-    MSC_HALO_ATTR(4, double)
-    MSC_HALO_ATTR(8, double)
-#undef MSC_HALO_ATTR
+    MSC_CUDA((halo_attributes<float, 0>()));
+    MSC_CUDA((halo_attributes<float, 1>()));
+    MSC_CUDA((halo_attributes<float, 2>()));
+    MSC_CUDA((halo_attributes<double, 0>()));
+    MSC_CUDA((halo_attributes<double, 1>()));
+    MSC_CUDA((halo_attributes<double, 2>()));
     MSC_CUDA(cudaFuncSetAttribute(msc::k_residual_diag, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)smem_residual(msc::kMaxNz)));
     MSC_CUDA(cudaFuncSetAttribute(msc::k_coupling<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1473,7 +1481,8 @@ void apply_tc_width(msc_plan *p, int N, int G = 1)
 // Autotuner front end: reuse the choices of an earlier plan of the same
 // shape (same sizes, batch, tap reach and options), else measure.
 // MSC_TUNE="c64=K,c32=K,bi=N[,bg=G]" fixes the choices (K: 0 neighbour
-// table, 1 halo 8 y/thread, 2 halo 4 y/thread; N: tcgen05 tile width,
+// table, 1 / 2 halo tiles with one / two threads per patch column, 3 to 5 separable
+// over channel boxes; N: tcgen05 tile width,
 // 0 = SIMT; G: 1 or 2 warp groups in the tcgen05 kernel, default 1).
 // Profiling runs use it so that a profiler's overhead cannot change what the
 // autotuner picks.
@@ -1858,7 +1867,7 @@ msc_status finalize(msc_plan *p)
     tm.mark("row tables (device)");
     {
         // Halo-tiled coupling: signed tap reach, tap window, position->row
-        // tables and the list of 8 x kHaloBX position patches that hold
+        // tables and the list of position patches that hold
         // channels of each system.
         int hx = 0, hy = 0;
         std::vector<std::pair<int, int>> sgn(p->K);
@@ -1872,9 +1881,7 @@ msc_status finalize(msc_plan *p)
         }
         int hyt = 1;
         while (hyt < hy) hyt <<= 1;
-        p->use_halo = (hx <= 8 && hyt <= 8 &&
-                       halo_smem(hx, hyt, 16, sizeof(double2)) <= 225 * 1024 &&
-                       halo_smem(hx, hyt, 32, sizeof(float2)) <= 225 * 1024);
+        p->use_halo = hx <= 8 && hyt <= 8;
         if (p->use_halo) {
             p->halo_hx = hx;
             p->halo_hy = hyt;
@@ -1882,22 +1889,29 @@ msc_status finalize(msc_plan *p)
             std::vector<int> win((size_t)(2 * hx + 1) * wy, -1);
             for (int t = 0; t < p->K; ++t)
                 win[(size_t)(sgn[t].first + hx) * wy + (sgn[t].second + hyt)] = t;
-            std::vector<int> wl;
-            const int nbx = (p->nkx + kHaloBX - 1) / kHaloBX, nby = (p->nky + 7) / 8;
-            for (int s2 = 0; s2 < p->B; ++s2) {
-                const SystemHost &sh = p->sys[s2];
-                std::vector<char> occ((size_t)nbx * nby, 0);
-                for (int j = 0; j < sh.C; ++j)
-                    occ[(size_t)(sh.ix[j] / kHaloBX) * nby + sh.iy[j] / 8] = 1;
-                for (int bx = 0; bx < nbx; ++bx)
-                    for (int by = 0; by < nby; ++by)
-                        if (occ[(size_t)bx * nby + by]) {
-                            wl.push_back(s2);
-                            wl.push_back(bx * kHaloBX);
-                            wl.push_back(by * 8);
-                        }
+            std::vector<int4> wl;
+            // The torus in as few patches of at most 8 x 16 (two segments) or 8 x 8 as
+            // cover it, of even size.
+            for (int seg = 2; seg >= 1; --seg) {
+                wl.clear();
+                const int nbx = (p->nkx + msc::kHaloMax - 1) / msc::kHaloMax;
+                const int nby = (p->nky + seg * msc::kHaloMax - 1) / (seg * msc::kHaloMax);
+                const int bw = (p->nkx + nbx - 1) / nbx, bh = (p->nky + nby - 1) / nby;
+                for (int s2 = 0; s2 < p->B; ++s2) {
+                    const SystemHost &sh = p->sys[s2];
+                    std::vector<char> occ((size_t)nbx * nby, 0);
+                    for (int j = 0; j < sh.C; ++j) occ[(size_t)(sh.ix[j] / bw) * nby + sh.iy[j] / bh] = 1;
+                    for (int bx = 0; bx < nbx; ++bx)
+                        for (int by = 0; by < nby; ++by)
+                            if (occ[(size_t)bx * nby + by]) wl.push_back(make_int4(s2, bx * bw, by * bh, 0));
+                }
+                p->halo_bx = bw;
+                p->halo_by = bh;
+                p->halo_seg = seg;
+                const int lines = (n + msc::halo_zc<double>() - 1) / msc::halo_zc<double>();
+                if ((int64_t)wl.size() * lines >= 3 * 148 && bh > msc::kHaloMax) break;
             }
-            p->nwork = (int)(wl.size() / 3);
+            p->nwork = (int)wl.size();
             MSC_CUDA(upload(p->tap_window, win));
             MSC_CUDA(upload(p->work, wl));
             separable_factors(p, win);
