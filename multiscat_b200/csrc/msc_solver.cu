@@ -1386,7 +1386,7 @@ msc_status setup_tensor_core(msc_plan *p)
         const size_t kpc = (size_t)(n + 15) / 16 * 16;
         cudaFuncAttributes fa{};
         p->tcc_smem = 4 * kpc * kpc + 512 * kpc + 1024;
-        p->tcc_ok = kpc <= 256 &&
+        p->tcc_ok = kpc <= msc::tc::kTccMaxKp &&
                     cudaFuncGetAttributes(&fa, msc::tc::k_block_inverse_tcc) == cudaSuccess &&
                     p->tcc_smem + fa.sharedSizeBytes <= (size_t)optin;
         if (p->tcc_ok) {
@@ -1591,26 +1591,27 @@ msc_status autotune_measure(msc_plan *p)
             });
             p->tune_log.push_back({"block_inverse32_simt_us", t_simt});
             p->use_tc = true;
-            // (the channel-major form, MSC_TUNE bg=3, is left out: 243 against
-            // 250 us per full-batch launch on the 512-beam cfg2 batch, but the
-            // batch was not faster end to end with it)
-            for (int G = 1; G <= (stream ? 1 : 2); ++G)
-                for (int N = stream ? 64 : 16; N <= (G == 1 ? best_n0 : p->tc2_max); N *= 2) {
-                    apply_tc_width(p, N, G);
-                    if (stream && p->tc_n != N) continue;    // does not fit at this width
-                    const float t = time_launch(p, [&](cudaStream_t st) {
-                        launch_block_inverse_t<float>(p, nullptr, a, b, 0, st);
-                    });
-                    p->tune_log.push_back({std::string("block_inverse32_tc") +
-                                               (stream ? "_stream" : G == 2 ? "2" : "") +
-                                               "_N" + std::to_string(N) + "_us",
-                                           t});
-                    if (best_n == 0 || t < best_t) {
-                        best_n = N;
-                        best_g = G;
-                        best_t = t;
-                    }
+            // widths of both group counts (2: no wider than tc2_max), then the
+            // channel-major form: the fastest where its 64-channel tiles fill the SMs
+            // (119409 x 150: 157 us against 212 at N = 128; 6760 x 131: 18 against
+            // 19), the narrow widths below that (1681 x 200 at N = 32: 18)
+            auto measure = [&](int N, int G, const std::string &name) {
+                apply_tc_width(p, N, G);
+                if (stream && p->tc_n != N) return;          // does not fit at this width
+                const float t = time_launch(p, [&](cudaStream_t st) {
+                    launch_block_inverse_t<float>(p, nullptr, a, b, 0, st);
+                });
+                p->tune_log.push_back({"block_inverse32_" + name + "_us", t});
+                if (best_n == 0 || t < best_t) {
+                    best_n = N;
+                    best_g = G;
+                    best_t = t;
                 }
+            };
+            for (int G = 1; G <= (stream ? 1 : 2); ++G)
+                for (int N = stream ? 64 : 16; N <= (G == 1 ? best_n0 : p->tc2_max); N *= 2)
+                    measure(N, G, (stream ? "tc_stream_N" : G == 2 ? "tc2_N" : "tc_N") + std::to_string(N));
+            if (!stream && p->tcc_ok) measure(128, kTcChannelMajor, "tcc");
             int tc_err = 0;
             MSC_CUDA(cudaMemcpy(&tc_err, p->tc_error.p, sizeof(int), cudaMemcpyDeviceToHost));
             if (tc_err) return fail(MSC_ERR_CUDA, "tensor-core block inverse timed out during tuning");

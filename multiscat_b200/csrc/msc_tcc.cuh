@@ -15,8 +15,18 @@
 // (no warp butterfly), and pkd is one value per thread.  The same E image
 // (8x8 core matrices: 8 rows of z, 8 consecutive k per 16-byte row) serves
 // both B operands, as in k_block_inverse_tc; the A buffer takes the x tile,
-// then yt, then (as raw FP32 rows) the next tile's x by one bulk copy.
-// TMEM: D1 at columns [0, kp), D2 at [256, 256 + kp).
+// then yt, then u as rows of global memory (one bulk store), then the next
+// tile's x (one bulk copy; its lines are asked into L2 when the tile is known).
+// TMEM: D1 at columns [0, kp); [256, 256 + kp) holds 1 / (pkd + lam), then D2.
+//
+// What bounds it: the phases of a tile run one after another, since E and one A
+// buffer fill the shared memory.  At n = 150, cycles per 64-channel tile: store and
+// copy with the inverses beside them 4500, staging 2600, GEMMs 2 x 2950 (2460 at the
+// tensor cores' rate), sums 2700, yt 2100, u 2050.  The same phases were 32700 when each
+// epilogue formed the inverses anew (FP64 sum, conversion and reciprocal, about 60
+// cycles of a warp each) and every lane stored its own row.  119409 x 150 (512 beams):
+// 243 -> 157 us per launch, against 212 us for the node-major form at N = 128 and
+// 44 us for the bytes alone.
 //
 // BF16x3 products (A_hi B_hi + A_hi B_lo + A_lo B_hi), FP32 accumulation,
 // pkd + lam in FP64 and the SFU reciprocal, every mbarrier wait bounded: on
@@ -29,19 +39,44 @@
 namespace msc {
 namespace tc {
 
-// 16 accumulator columns of this warp's 32 lanes, waited for.
-__device__ __forceinline__ void tmem_ld16f(uint32_t taddr, float (&v)[16])
+// 8 accumulator columns of this warp's 32 lanes, not waited for.
+__device__ __forceinline__ void tmem_ld8_nowait(uint32_t taddr, uint32_t (&r)[8])
 {
-    uint32_t r[16];
-    tmem_ld16_nowait(taddr, r);
-    tmem_wait_ld();
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
 }
+
+// 8 accumulator columns of this warp's 32 lanes, written; completed by tmem_wait_st.
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const float (&v)[8])
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "f"(v[0]),
+                 "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// Bulk copy shared -> global of this thread's bulk group; bytes and both addresses are
+// multiples of 16.
+__device__ __forceinline__ void bulk_s2g(void *dst, const void *src, uint32_t bytes)
+{
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)),
+                 "r"(bytes)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void bulk_prefetch_l2(const void *src, uint32_t bytes)
+{
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
+
+// Largest kp (what the shared memory takes), and the units of 8 accumulator columns
+// that a warp reads from TMEM at a time.
+constexpr int kTccMaxKp = 176, kTccBatch = 1;
 
 // One CTA per SM, 512 threads: warp w reads TMEM lanes 32 (w % 4) .. + 31
 // (rows c, i.e. 16 channels) and the column group w / 4 (a quarter of kp,
-// in 16-column chunks).
+// in 8-column units).
 __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tcc(TcParams prm)
 {
     constexpr int TR = 64;                    // channels per tile
@@ -51,8 +86,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tcc(TcParams prm)
     __shared__ __align__(8) uint64_t bar_e, bar_mma, bar_pf;
     __shared__ uint32_t tmem_base_s;
     __shared__ double sm_part[4][ROWS];       // Sherman-Morrison partial sums [column group][row]
-    __shared__ float2 beta_s[TR];
-    __shared__ double pkd_s[TR];
     __shared__ double2 cf_s[TR];              // c_j / (1 - c_j fn_j)
     __shared__ double lam_s[256];
     __shared__ float en_s[256];
@@ -62,8 +95,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tcc(TcParams prm)
     const int lq = warp & 3, cg = warp >> 2;
     const int n = prm.n, kp = prm.kp;
     const int kb = kp >> 3;                               // 8-blocks along z and k
-    const int nch = kp >> 4;                              // 16-column chunks of an accumulator
-    const int ch0 = (cg * nch) >> 2, ch1 = ((cg + 1) * nch) >> 2;   // this warp's chunks
+    const int u0 = (cg * kb) >> 2, nu = (((cg + 1) * kb) >> 2) - u0;   // this warp's 8-column units
     const uint32_t part_bytes = (uint32_t)kp * kp * 2u;   // one of E_hi / E_lo
     unsigned char *e_hi = smem;
     unsigned char *e_lo = smem + part_bytes;
@@ -139,6 +171,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tcc(TcParams prm)
     const bool use_pf = (n % 2 == 0) && upt <= kMaxPf &&
                         (reinterpret_cast<uintptr_t>(prm.x) & 15u) == 0;
     float2 *raw = reinterpret_cast<float2 *>(a_hi);
+    // the result leaves through the same buffer, as one bulk store per tile
+    const bool bulk_out = (n % 2 == 0) && (reinterpret_cast<uintptr_t>(prm.out) & 15u) == 0;
     auto prefetch = [&](int t) {
         if (tid == 0) {
             const int r0 = t * TR, nr = min(TR, prm.rows - r0);
@@ -162,15 +196,47 @@ __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tcc(TcParams prm)
     __syncthreads();
     int tile = next_s;
     __syncthreads();            // every thread has read next_s before the loop rewrites it
-    if (use_pf && tile < prm.ntiles) prefetch(tile);
+    bool pf_due = use_pf && tile < prm.ntiles;     // the tile's copy is still to be started
 
     while (tile < prm.ntiles && ok) {
         const int row0 = tile * TR;
         const int nrow = min(TR, prm.rows - row0);
-        for (int j = tid; j < TR; j += kThreads) {
-            const bool in = j < nrow;
-            pkd_s[j] = in ? prm.row_pkd[row0 + j] : 0.0;
-            cf_s[j] = in ? prm.row_cf[row0 + j] : make_double2(0.0, 0.0);
+        for (int j = tid; j < TR; j += kThreads)
+            cf_s[j] = j < nrow ? prm.row_cf[row0 + j] : make_double2(0.0, 0.0);
+        // 1 / (pkd_j + lam_k) of this thread's columns, for both epilogues, while the tile
+        // arrives (the MMAs keep the shared memory busy: formed under GEMM 1 they took
+        // twice as long); the two lanes of a channel (re, im) form half of them each.
+        // They wait in the columns of D2, which this warp has read and GEMM 2 writes only
+        // later (in registers they spilled).  Zero past the tile's rows and the nodes, so
+        // that the epilogues need no tests.
+        const bool row_ok = jc < nrow;
+        const int part = c & 1;
+        const uint32_t lane_base = (uint32_t)(lq * 32) << 16;
+        const uint32_t t1 = d1 + lane_base + (uint32_t)(8 * u0), t2 = d2 + lane_base + (uint32_t)(8 * u0);
+        {
+            const double pkd_j = row_ok ? prm.row_pkd[row0 + jc] : 0.0;
+            auto unit = [&](int u) {
+                float inv[8];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int k = 8 * (u0 + u) + 4 * part + e;
+                    const float mine = row_ok && k < n ? shifted_inverse(pkd_j, lam_s[k]) : 0.f;
+                    const float other = __shfl_xor_sync(0xffffffffu, mine, 1);
+                    inv[e] = part ? other : mine;
+                    inv[4 + e] = part ? mine : other;
+                }
+                tmem_st8(t2 + (uint32_t)(8 * u), inv);
+            };
+            // the buffer is free once the last tile's store has read it, about two units on
+            const int first = min(nu, 2);
+            for (int u = 0; u < first; ++u) unit(u);
+            if (pf_due) {
+                if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                prefetch(tile);
+                pf_due = false;
+            }
+            for (int u = first; u < nu; ++u) unit(u);
+            tmem_wait_st();
         }
 
         // ---- stage x as the A operand of GEMM 1 (K-major: rows = 2 TR re/im, K = z)
@@ -240,7 +306,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tcc(TcParams prm)
         }
         // the next active tile is found by warp 1 while the MMAs run; every
         // thread read next_s before the previous tile's last barrier
-        if (tid == 32) next_s = find_active(tile + gridDim.x);
+        if (tid == 32) {
+            const int t = find_active(tile + gridDim.x);
+            next_s = t;
+            if (use_pf && t < prm.ntiles)
+                bulk_prefetch_l2(prm.x + (size_t)t * TR * n, (uint32_t)min(TR, prm.rows - t * TR) * (uint32_t)n * 8u);
+        }
         mma_pending = true;
         if (mbar_wait(&bar_mma, mma_phase)) {
             mma_phase ^= 1u;
@@ -251,10 +322,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tcc(TcParams prm)
         tc_fence_after();
         if (!__syncthreads_and(ok)) { ok = false; break; }
 
-        const bool row_ok = jc < nrow;
-        const int part = c & 1;
-        const double pkd_j = pkd_s[jc];
-        const uint32_t lane_base = (uint32_t)(lq * 32) << 16;
 
         // ---- epilogue 1a: Sherman-Morrison partial sums over this warp's
         // columns, s_c = sum_k en_k D1[c, k] / (pkd_j + lam_k)
@@ -262,62 +329,71 @@ __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tcc(TcParams prm)
             // (the thread's sum runs in FP64: its ~kp/4 terms come in sequence,
             // not as a tree, and near a resonance of H0 + pkd they cancel)
             double sacc = 0.0;
-            for (int q = ch0; q < ch1; ++q) {
-                float v[16];
-                tmem_ld16f(d1 + lane_base + (uint32_t)(16 * q), v);
+#pragma unroll 1
+            for (int ub = 0; ub < nu; ub += kTccBatch) {
+                uint32_t r[kTccBatch][8], w[kTccBatch][8];
 #pragma unroll
-                for (int e = 0; e < 16; ++e) {
-                    const int k = 16 * q + e;
-                    // select, not multiply: columns past n carry nothing
-                    if (k < n) sacc = fma((double)(en_s[k] * shifted_inverse(pkd_j, lam_s[k])), (double)v[e], sacc);
+                for (int q = 0; q < kTccBatch; ++q)
+                    if (ub + q < nu) {
+                        tmem_ld8_nowait(t1 + (uint32_t)(8 * (ub + q)), r[q]);
+                        tmem_ld8_nowait(t2 + (uint32_t)(8 * (ub + q)), w[q]);
+                    }
+                tmem_wait_ld();
+#pragma unroll
+                for (int q = 0; q < kTccBatch; ++q) {
+                    if (ub + q >= nu) continue;
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        const float we = en_s[8 * (u0 + ub + q) + e] * __uint_as_float(w[q][e]);
+                        sacc = fma((double)we, (double)__uint_as_float(r[q][e]), sacc);
+                    }
                 }
             }
-            sm_part[cg][c] = row_ok ? sacc : 0.0;
-        }
-        __syncthreads();
-        for (int j = tid; j < TR; j += kThreads) {
-            double2 b = make_double2(0.0, 0.0);
-            if (j < nrow) {
-                double sr = 0.0, si = 0.0;   // fixed summation order: deterministic
-                for (int w = 0; w < 4; ++w) {
-                    sr += sm_part[w][2 * j];
-                    si += sm_part[w][2 * j + 1];
-                }
-                b = cmul(cf_s[j], make_double2(sr, si));
-            }
-            beta_s[j] = make_float2((float)b.x, (float)b.y);
+            sm_part[cg][c] = sacc;
         }
         __syncthreads();
 
         // ---- epilogue 1b: yt[c, k] = (D1[c, k] + beta_j en_k) / (pkd_j + lam_k)
         // as the K-major A operand of GEMM 2 (one row per thread, 8 k per
-        // 16-byte unit; columns past n are zero)
+        // 16-byte unit; columns past n are zero); every thread forms its channel's beta
         {
-            const float bpart = part ? beta_s[jc].y : beta_s[jc].x;
-            for (int q = ch0; q < ch1; ++q) {
-                float v[16];
-                tmem_ld16f(d1 + lane_base + (uint32_t)(16 * q), v);
-                uint32_t hw[8], lw[8];
+            double sr = 0.0, si = 0.0;       // fixed summation order: deterministic
 #pragma unroll
-                for (int e = 0; e < 16; e += 2) {
-                    const int k = 16 * q + e;
-                    float y0 = 0.f, y1 = 0.f;
-                    if (row_ok && k < n)
-                        y0 = (v[e] + bpart * en_s[k]) * shifted_inverse(pkd_j, lam_s[k]);
-                    if (row_ok && k + 1 < n)
-                        y1 = (v[e + 1] + bpart * en_s[k + 1]) * shifted_inverse(pkd_j, lam_s[k + 1]);
-                    const __nv_bfloat162 h = __floats2bfloat162_rn(y0, y1);
-                    const float2 fh = __bfloat1622float2(h);
-                    const __nv_bfloat162 l = __floats2bfloat162_rn(y0 - fh.x, y1 - fh.y);
-                    hw[e >> 1] = *reinterpret_cast<const uint32_t *>(&h);
-                    lw[e >> 1] = *reinterpret_cast<const uint32_t *>(&l);
+            for (int w = 0; w < 4; ++w) {
+                sr += sm_part[w][2 * jc];
+                si += sm_part[w][2 * jc + 1];
+            }
+            const double2 b = cmul(cf_s[jc], make_double2(sr, si));
+            const float bpart = (float)(part ? b.y : b.x);
+#pragma unroll 1
+            for (int ub = 0; ub < nu; ub += kTccBatch) {
+                uint32_t r[kTccBatch][8], w[kTccBatch][8];
+#pragma unroll
+                for (int q = 0; q < kTccBatch; ++q)
+                    if (ub + q < nu) {
+                        tmem_ld8_nowait(t1 + (uint32_t)(8 * (ub + q)), r[q]);
+                        tmem_ld8_nowait(t2 + (uint32_t)(8 * (ub + q)), w[q]);
+                    }
+                tmem_wait_ld();
+#pragma unroll
+                for (int q = 0; q < kTccBatch; ++q) {
+                    if (ub + q >= nu) continue;
+                    const int k0 = 8 * (u0 + ub + q);
+                    uint32_t hw[4], lw[4];
+#pragma unroll
+                    for (int e = 0; e < 8; e += 2) {
+                        const float y0 = (__uint_as_float(r[q][e]) + bpart * en_s[k0 + e]) * __uint_as_float(w[q][e]);
+                        const float y1 = (__uint_as_float(r[q][e + 1]) + bpart * en_s[k0 + e + 1]) * __uint_as_float(w[q][e + 1]);
+                        const __nv_bfloat162 h = __floats2bfloat162_rn(y0, y1);
+                        const float2 fh = __bfloat1622float2(h);
+                        const __nv_bfloat162 l = __floats2bfloat162_rn(y0 - fh.x, y1 - fh.y);
+                        hw[e >> 1] = *reinterpret_cast<const uint32_t *>(&h);
+                        lw[e >> 1] = *reinterpret_cast<const uint32_t *>(&l);
+                    }
+                    const uint32_t o = kmaj_off(c, k0, ROWS);
+                    *reinterpret_cast<uint4 *>(a_hi + o) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+                    *reinterpret_cast<uint4 *>(a_lo + o) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
                 }
-                const int k0 = 16 * q;
-                const uint32_t o0 = kmaj_off(c, k0, ROWS), o1 = kmaj_off(c, k0 + 8, ROWS);
-                *reinterpret_cast<uint4 *>(a_hi + o0) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-                *reinterpret_cast<uint4 *>(a_hi + o1) = make_uint4(hw[4], hw[5], hw[6], hw[7]);
-                *reinterpret_cast<uint4 *>(a_lo + o0) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
-                *reinterpret_cast<uint4 *>(a_lo + o1) = make_uint4(lw[4], lw[5], lw[6], lw[7]);
             }
         }
         tc_fence_before();
@@ -348,49 +424,69 @@ __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tcc(TcParams prm)
         }
         tc_fence_after();
         if (!__syncthreads_and(ok)) { ok = false; break; }
-        // the A buffer is free: start the next tile's copy
         const int next = next_s;
-        if (use_pf && next < prm.ntiles) prefetch(next);
 
-        // ---- epilogue 2: u rows to global.  Lanes 2i and 2i + 1 hold the re
-        // and im rows of one channel; one shuffle per pair of values gives
-        // each lane 8 complex values of consecutive z (the even lane the
-        // chunk's first half), stored as 16-byte pairs where aligned.
-        {
-            const bool odd = lane & 1;
-            float2 *orow = prm.out + (size_t)(row0 + jc) * n;
-            const bool pairs = (n % 2 == 0) && (reinterpret_cast<uintptr_t>(prm.out) & 15u) == 0;
-            for (int q = ch0; q < ch1; ++q) {
-                float v[16];
-                tmem_ld16f(d2 + lane_base + (uint32_t)(16 * q), v);
-                float2 o[8];
+        // ---- epilogue 2: u rows to global.  The A buffer is free: the tile's rows are
+        // laid out there as in global memory and leave by one bulk store (a thread's own
+        // stores, 16 bytes of another row per lane, took 6000 cycles a tile against 2000);
+        // the next tile's copy starts once it has read them.
+        // (Lanes 2i and 2i + 1 hold re and im of a channel: one exchange gives each four
+        // whole values of a unit.)
+        float2 *urow = raw + (size_t)jc * n;
+#pragma unroll 1
+        for (int ub = 0; ub < nu; ub += kTccBatch) {
+            uint32_t r[kTccBatch][8];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float send = odd ? v[i] : v[8 + i];
-                    const float recv = __shfl_xor_sync(0xffffffffu, send, 1);
-                    o[i] = odd ? make_float2(recv, v[8 + i]) : make_float2(v[i], recv);
+            for (int q = 0; q < kTccBatch; ++q)
+                if (ub + q < nu) tmem_ld8_nowait(t2 + (uint32_t)(8 * (ub + q)), r[q]);
+            tmem_wait_ld();
+#pragma unroll
+            for (int q = 0; q < kTccBatch; ++q) {
+                if (ub + q >= nu) continue;
+                const int z = 8 * (u0 + ub + q) + 4 * part;
+                float2 o[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float a = __uint_as_float(r[q][i]), b = __uint_as_float(r[q][4 + i]);
+                    const float recv = __shfl_xor_sync(0xffffffffu, part ? a : b, 1);
+                    o[i] = part ? make_float2(recv, b) : make_float2(a, recv);
                 }
-                const int zb = 16 * q + (odd ? 8 : 0);
                 if (!row_ok) continue;
-                if (pairs) {
+                if ((n & 1) == 0) {
 #pragma unroll
-                    for (int i = 0; i < 8; i += 2)
-                        if (zb + i < n)
-                            *reinterpret_cast<float4 *>(orow + zb + i) =
+                    for (int i = 0; i < 4; i += 2)
+                        if (z + i < n)
+                            *reinterpret_cast<float4 *>(urow + z + i) =
                                 make_float4(o[i].x, o[i].y, o[i + 1].x, o[i + 1].y);
                 } else {
 #pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        if (zb + i < n) orow[zb + i] = o[i];
+                    for (int i = 0; i < 4; ++i)
+                        if (z + i < n) urow[z + i] = o[i];
                 }
             }
         }
         tc_fence_before();
-        __syncthreads();
+        if (bulk_out) {
+            fence_proxy_async();
+            __syncthreads();
+            if (tid == 0) bulk_s2g(prm.out + (size_t)row0 * n, raw, (uint32_t)nrow * (uint32_t)n * 8u);
+            if (!use_pf) {                          // read before it is staged anew
+                if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                __syncthreads();
+            }
+        } else {
+            __syncthreads();
+            float2 *o = prm.out + (size_t)row0 * n;
+            for (int i = tid; i < nrow * n; i += kThreads) o[i] = raw[i];
+            fence_proxy_async();
+            __syncthreads();
+        }
+        pf_due = use_pf && next < prm.ntiles;
         tile = next;
     }
 
     if (!ok && tid == 0 && prm.error) atomicExch(prm.error, 1);
+    if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     // Drain on a time-out: no copy may land and no MMA may write after the
     // kernel frees its TMEM and leaves (each wait bounded).
     if (tid == 0 && pf_pending) (void)mbar_wait(&bar_pf, pf_phase);
