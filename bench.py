@@ -195,8 +195,8 @@ def kernel_records(kt: dict, res, n: int, taps: int, mixed: bool, dcgs: bool, te
       x3 for the BF16x3 split on tcgen05 (bound: tensor; else the FMA pipe);
     coupling: 8 K n flop per row (K taps, one complex MAC each), ~27 flop per
       byte at K = 80, so the FMA pipe bounds it, not HBM; the separable form
-      (sep = (hx, HY) of its window) does 8 ((2hx+1)(8+2HY)/8 + 2HY + 2) n
-      flop per row, which leaves its FMA and HBM roofs close: the line names
+      (sep = (hx, HY) of its window) does 8 ((2hx+1) + (2HY+1) + 1) n flop per
+      row, which leaves its FMA and HBM roofs close: the line names
       the tighter one;
     Arnoldi passes: HBM bytes, one read or write of a row of a Krylov vector
       per vector touched: DCGS2 reduction (j + 1) + 1 reads at step j, update
@@ -232,7 +232,7 @@ def kernel_records(kt: dict, res, n: int, taps: int, mixed: bool, dcgs: bool, te
                         "rows": r_done, "bytes": 2.0 * es * n * r_done})
         elif k == "coupling" and sep:
             hx, hy = sep
-            per_row = 8.0 * ((2 * hx + 1) * (8 + 2 * hy) / 8.0 + 2 * hy + 2) * n
+            per_row = 8.0 * ((2 * hx + 1) + (2 * hy + 1) + 1) * n
             fl = per_row * steps_rows
             nbytes = 3.0 * es * n * steps_rows
             if fl / (fma_peak * 1e12) >= nbytes / (hbm * 1e9):
@@ -337,7 +337,7 @@ def run_b200(args) -> None:
     taps = plan.n_taps
     peaks, peak_kind = load_peaks()
     fma = measure_fma_peaks()
-    tensor = mixed and "tc_" in tuning.get("chosen", "")
+    tensor = mixed and "block_inverse32=tc" in tuning.get("chosen", "")
     chosen = tuning.get("chosen", "")
     sep = None
     if ("coupling32=separable" if mixed else "coupling64=separable") in chosen:

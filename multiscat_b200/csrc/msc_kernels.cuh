@@ -16,8 +16,8 @@
 //
 // The Krylov kernels are templated on the vector precision R: double for the
 // plain FP64 solve, float for the inner solve of the mixed form.  Reductions
-// (dot products, norms) always accumulate in FP64 and the GMRES scalars
-// (Hessenberg, Givens, g) are FP64.
+// (dot products, norms) accumulate in FP64 (in the FP32 inner solve after partial sums
+// of a few terms in a lane) and the GMRES scalars (Hessenberg, Givens, g) are FP64.
 #pragma once
 
 #include "msc_common.cuh"

@@ -1593,8 +1593,8 @@ msc_status autotune_measure(msc_plan *p)
             p->use_tc = true;
             // widths of both group counts (2: no wider than tc2_max), then the
             // channel-major form: the fastest where its 64-channel tiles fill the SMs
-            // (119409 x 150: 157 us against 212 at N = 128; 6760 x 131: 18 against
-            // 19), the narrow widths below that (1681 x 200 at N = 32: 18)
+            // (119409 x 150: 157 us against 210 at N = 128), the narrow widths below
+            // that (1681 x 200: 16 at N = 32, in 106 tiles instead of 27)
             auto measure = [&](int N, int G, const std::string &name) {
                 apply_tc_width(p, N, G);
                 if (stream && p->tc_n != N) return;          // does not fit at this width

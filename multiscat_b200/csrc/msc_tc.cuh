@@ -33,10 +33,14 @@
 // on time-out the kernel records an error code, stops issuing work and still
 // releases its TMEM.
 //
-// The epilogues are chains of short dependent steps (TMEM load, FP64 sum
-// and SFU reciprocal, shuffles); 16 warps keep four per scheduler to hide
-// them, with at most 128 registers per thread (the accumulator is read 32
-// columns at a time).
+// The epilogues are chains of short dependent steps (TMEM load, products,
+// shuffles); 16 warps keep four per scheduler to hide them, with at most 128
+// registers per thread (the accumulator is read 16 columns at a time).  The
+// values 1 / (pkd + lam) that both need are formed once per tile, while its
+// rows arrive, by all warps, and wait in TMEM: us per launch, formed by each
+// epilogue -> once: 1681 x 200 at N = 32 19.5 -> 16.0, 119409 x 150 at N = 32
+// 598 -> 482, N = 64 345 -> 306, N = 128 212 -> 210 (there the MMAs, whose A
+// operand makes every one of them cost about 70 cycles, and the serial phases).
 //
 // Warp groups.  With G = 2 the 16 warps form two groups of 8 (each group's
 // warps cover the four TMEM lane quarters and two column halves); each group has
@@ -140,6 +144,27 @@ __device__ __forceinline__ void tmem_ld_chunks(uint32_t taddr, int nch, float (&
 #pragma unroll
         for (int i = 0; i < 16; ++i) v[q][i] = __uint_as_float(r[q][i]);
 }
+
+// 8 accumulator columns of this warp's 32 lanes, not waited for.
+__device__ __forceinline__ void tmem_ld8_nowait(uint32_t taddr, uint32_t (&r)[8])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+}
+
+// 2 or 8 accumulator columns of this warp's 32 lanes, written; completed by tmem_wait_st.
+__device__ __forceinline__ void tmem_st2(uint32_t taddr, float a, float b)
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1,%2};" ::"r"(taddr), "f"(a), "f"(b) : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const float (&v)[8])
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "f"(v[0]),
+                 "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // Shared-memory matrix descriptor (no swizzle, canonical 8x16-byte core matrices).
 __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes)
@@ -267,7 +292,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tc(TcParams prm)
     __shared__ uint32_t tmem_base_s;
     __shared__ float sm_part[G][4][2][N];     // Sherman-Morrison partial sums [group][lane quarter][M tile][col]
     __shared__ float2 beta_s[G][TR];
-    __shared__ double pkd_s[G][TR];
     __shared__ double2 cf_s[G][TR];            // the tile's c_j / (1 - c_j fn_j), loaded with pkd
     __shared__ double lam_s[256];             // eigenvalues of H0 (k < n <= 256), 0 past n
     __shared__ float en_s[256];               // last components E[n-1, k] (FP32), 0 past n
@@ -280,8 +304,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tc(TcParams prm)
     constexpr int NCG = NW / 4;                           // column groups (warps per lane quarter)
     constexpr int CW = (N / NCG >= 16) ? N / NCG : 16;    // columns per warp
     const int c_begin = (wl >> 2) * CW;
-    constexpr bool kInvCache = CW == 16 * kLdChunks;      // one TMEM pass per M tile
-    float invc[2][kInvCache ? CW / 2 : 1];                // 1 / (pkd_j + lam_k) of epilogue 1a
+    constexpr int JW = TR / NCG;                          // channels per warp, of the inverses
     const bool epi = c_begin < N;                         // narrow tiles: surplus column groups sit out
     const int n = prm.n, kp = prm.kp, mt_count = prm.mt;
     const int kb = kp >> 3;                               // 8-blocks along z and k
@@ -400,8 +423,37 @@ __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tc(TcParams prm)
         const int nrow = min(TR, prm.rows - row0);
         for (int j = gtid; j < TR; j += GT) {
             const bool in = j < nrow;
-            pkd_s[g][j] = in ? prm.row_pkd[row0 + j] : 0.0;
             cf_s[g][j] = in ? prm.row_cf[row0 + j] : make_double2(0.0, 0.0);
+        }
+
+        // ---- 1 / (pkd_j + lam_k) for both epilogues, while the tile arrives: a warp
+        // forms its lane quarter's k for JW channels, all 16 warps also at narrow N, and
+        // leaves them in the first TR columns of D2 of the M tile, which GEMM 2 writes
+        // only later (formed by each epilogue for itself, a sum in FP64, a conversion and
+        // a reciprocal cost about 60 cycles of a warp: half of both epilogues).  Zero for
+        // channels past the tile and k past the nodes.
+        {
+            tc_fence_after();                  // the last tile's reads of D2
+            const int j0 = (wl >> 2) * JW;
+            const uint32_t lanes = (uint32_t)(lq * 32) << 16;
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                if (m >= mt_count || m * 128 + lq * 32 >= n) break;
+                const int k = m * 128 + lq * 32 + lane;
+                const double lam_k = lam_s[k];
+                const uint32_t dst = tmem + lanes + (uint32_t)((mt_count + m) * N + j0);
+#pragma unroll
+                for (int j = 0; j < JW; j += 2) {
+                    float iv[2];
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
+                        iv[e] = k < n && j0 + j + e < nrow
+                                    ? shifted_inverse(prm.row_pkd[row0 + j0 + j + e], lam_k) : 0.f;
+                    tmem_st2(dst + (uint32_t)j, iv[0], iv[1]);
+                }
+            }
+            tmem_wait_st();
+            tc_fence_before();
         }
 
         // ---- stage x as the B operand of GEMM 1 (K-major: rows = 2 TR re/im
@@ -496,45 +548,34 @@ __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tc(TcParams prm)
         // GEMM 2 consumes; pkd + lam in FP64).  Each 16-column chunk is
         // reduced over the warp's 32 k-lanes by a reduce-scatter butterfly
         // (16 shuffles), then over lane quarters and M tiles in a fixed order.
-        // With one TMEM pass per M tile (CW = 32) the thread keeps its
-        // 1 / (pkd_j + lam_k) values for epilogue 1b.
 #pragma unroll
         for (int m = 0; m < 2; ++m) {
             if (m >= mt_count || !epi) break;
             const int k = m * 128 + lq * 32 + lane;
+            if (m * 128 + lq * 32 >= n) {      // no node in these lanes
+                if (lane < 16)
+                    for (int c0 = c_begin; c0 < c_begin + CW; c0 += 16) sm_part[g][lq][m][c0 + lane] = 0.f;
+                continue;
+            }
             const bool valid = k < n;
-            const double lam_k = lam_s[k];
             const float en_k = en_s[k];
+            const uint32_t lanes = (uint32_t)(lq * 32) << 16;
 #pragma unroll
-            for (int cb = c_begin; cb < c_begin + CW; cb += 16 * kLdChunks) {
-            const int nch = min(kLdChunks, (c_begin + CW - cb) >> 4);
-            float vv[kLdChunks][16];
-            tmem_ld_chunks(tmem + ((uint32_t)(lq * 32) << 16) + (uint32_t)(m * N + cb), nch, vv);
+            for (int c0 = c_begin; c0 < c_begin + CW; c0 += 16) {
+                uint32_t r[16], w[8];
+                tmem_ld16_nowait(tmem + lanes + (uint32_t)(m * N + c0), r);
+                tmem_ld8_nowait(tmem + lanes + (uint32_t)((mt_count + m) * N + (c0 >> 1)), w);
+                tmem_wait_ld();
+                float v[16];
 #pragma unroll
-            for (int q = 0; q < kLdChunks; ++q) {
-                if (q >= nch) continue;
-                const int c0 = cb + 16 * q;
-                float (&v)[16] = vv[q];
-#pragma unroll
-                for (int c = 0; c < 16; c += 2) {
+                for (int c = 0; c < 16; ++c) {
                     // select, not multiply: accumulator rows k >= kp of the last
                     // M tile come from bytes past E in shared memory and may hold
                     // NaN, which a zero weight would not remove
-                    const int j = (c0 + c) >> 1;
-                    if (valid && j < nrow) {
-                        const float iv = shifted_inverse(pkd_s[g][j], lam_k);
-                        if constexpr (kInvCache) invc[m][(16 * q + c) >> 1] = iv;
-                        const float w = en_k * iv;
-                        v[c] *= w;
-                        v[c + 1] *= w;
-                    } else {
-                        v[c] = 0.f;
-                        v[c + 1] = 0.f;
-                    }
+                    v[c] = valid ? __uint_as_float(r[c]) * (en_k * __uint_as_float(w[c >> 1])) : 0.f;
                 }
                 const float sum = warp_reduce_scatter16(v, lane);
                 if ((lane & 1) == 0) sm_part[g][lq][m][c0 + ((lane >> 1) & 15)] = sum;
-            }
             }
         }
         group_sync(bar_id, GT);
@@ -560,35 +601,30 @@ __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tc(TcParams prm)
         // (rows k >= kp are never read; k in [n, kp) are zero).
 #pragma unroll
         for (int m = 0; m < 2; ++m) {
-            if (m >= mt_count || !epi) break;
+            if (m >= mt_count || !epi || m * 128 + lq * 32 >= kp) break;
             const int k = m * 128 + lq * 32 + lane;
-            const bool valid = k < n;
+            const bool valid = k < n, some = m * 128 + lq * 32 < n;
             const bool stage = k < kp;
-            const double lam_k = lam_s[k];
             const float en_k = en_s[k];
+            const uint32_t lanes = (uint32_t)(lq * 32) << 16;
 #pragma unroll
-            for (int cb = c_begin; cb < c_begin + CW; cb += 16 * kLdChunks) {
-            const int nch = min(kLdChunks, (c_begin + CW - cb) >> 4);
-            float vv[kLdChunks][16];
-            tmem_ld_chunks(tmem + ((uint32_t)(lq * 32) << 16) + (uint32_t)(m * N + cb), nch, vv);
-            if (!stage) continue;
-#pragma unroll
-            for (int q = 0; q < kLdChunks; ++q) {
-                if (q >= nch) continue;
-                const int c0 = cb + 16 * q;
-                const float (&v)[16] = vv[q];
+            for (int c0 = c_begin; c0 < c_begin + CW; c0 += 16) {
+                uint32_t r[16], w[8];
+                if (some) {
+                    tmem_ld16_nowait(tmem + lanes + (uint32_t)(m * N + c0), r);
+                    tmem_ld8_nowait(tmem + lanes + (uint32_t)((mt_count + m) * N + (c0 >> 1)), w);
+                    tmem_wait_ld();
+                }
+                if (!stage) continue;
                 uint32_t hw[8], lw[8];
 #pragma unroll
                 for (int c = 0; c < 16; c += 2) {
-                    const int j = (c0 + c) >> 1;
                     float yr = 0.f, yi = 0.f;
-                    if (valid && j < nrow) {
-                        float inv;
-                        if constexpr (kInvCache) inv = invc[m][(16 * q + c) >> 1];
-                        else inv = shifted_inverse(pkd_s[g][j], lam_k);
-                        const float2 b = beta_s[g][j];
-                        yr = (v[c] + b.x * en_k) * inv;
-                        yi = (v[c + 1] + b.y * en_k) * inv;
+                    if (valid) {
+                        const float inv = __uint_as_float(w[c >> 1]);
+                        const float2 b = beta_s[g][(c0 + c) >> 1];
+                        yr = (__uint_as_float(r[c]) + b.x * en_k) * inv;
+                        yi = (__uint_as_float(r[c + 1]) + b.y * en_k) * inv;
                     }
                     const __nv_bfloat162 h = __floats2bfloat162_rn(yr, yi);
                     const float2 fh = __bfloat1622float2(h);
@@ -602,7 +638,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tc(TcParams prm)
                 *reinterpret_cast<uint4 *>(b_hi + o + 128) = make_uint4(hw[4], hw[5], hw[6], hw[7]);
                 *reinterpret_cast<uint4 *>(b_lo + o) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
                 *reinterpret_cast<uint4 *>(b_lo + o + 128) = make_uint4(lw[4], lw[5], lw[6], lw[7]);
-            }
             }
         }
         tc_fence_before();

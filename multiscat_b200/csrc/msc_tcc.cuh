@@ -39,23 +39,6 @@
 namespace msc {
 namespace tc {
 
-// 8 accumulator columns of this warp's 32 lanes, not waited for.
-__device__ __forceinline__ void tmem_ld8_nowait(uint32_t taddr, uint32_t (&r)[8])
-{
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr));
-}
-
-// 8 accumulator columns of this warp's 32 lanes, written; completed by tmem_wait_st.
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const float (&v)[8])
-{
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "f"(v[0]),
-                 "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
 // Bulk copy shared -> global of this thread's bulk group; bytes and both addresses are
 // multiples of 16.
 __device__ __forceinline__ void bulk_s2g(void *dst, const void *src, uint32_t bytes)
