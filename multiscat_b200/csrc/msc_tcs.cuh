@@ -20,7 +20,12 @@
 // bounds it: E from L2, 128 kp^2 / N bytes per channel and product pair (n = 300,
 // N = 128: 11.6 KB a channel against 4.8 KB of x and u in HBM) and the phases
 // of a tile that follow one another (stage, product, sums, y, product, store).
-// Measured, 26244 rows x 300: 223 us (N = 128), 382 us (N = 64), CUDA cores 880 us.
+// While thread 0 feeds the ring, the other lanes of its warp wait at a warp barrier
+// and one lane of every other warp polls for the end of the product: with all 512
+// threads polling, thread 0 got to run half as often (a product took 50000 cycles
+// instead of 25000; 12800 are the MMAs).
+// Measured, 26244 rows x 300: 159 us (N = 128), 252 us (N = 64), before the single
+// polls 226 and 384, CUDA cores 880 us.
 // Like the resident form it is the `tensor_cores` option of a mixed plan
 // (autotuned unless the caller sets it); tensor_cores=False keeps FP32 products.
 // The solve's results do not change with it: the FP64 residual decides (|u - A psi|
@@ -65,6 +70,14 @@ struct TcStreamParams {
     TcParams t;                          // e_img unused
     const __nv_bfloat16 *img1, *img2;    // [piece][hi, lo][2 K blocks][kp / 8][8][8]
 };
+
+// mbar_wait by one lane for its warp: sixteen polls instead of 512.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, int lane)
+{
+    bool done = true;
+    if (lane == 0) done = mbar_wait(bar, parity);
+    return __shfl_sync(0xffffffffu, done, 0);
+}
 
 template <int N, int S>
 __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tcs(TcStreamParams sp)
@@ -235,6 +248,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tcs(TcStreamParam
             ok = run_product(idesc_mn, false);
             mma_commit(&bar_mma);
         }
+        __syncwarp();           // lanes that polled bar_mma meanwhile would hold thread 0 up
         // the next active tile, while the MMAs run (every thread read next_s
         // before the previous tile's last barrier); its rows go to L2
         if (tid == 32) {
@@ -249,7 +263,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tcs(TcStreamParam
                                  : "memory");
             }
         }
-        if (!mbar_wait(&bar_mma, mma_phase)) ok = false;
+        if (!mbar_wait_warp(&bar_mma, mma_phase, lane)) ok = false;
         mma_phase ^= 1u;
         tc_fence_after();
         if (!__syncthreads_and(ok)) { ok = false; break; }
@@ -351,7 +365,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tcs(TcStreamParam
             ok = run_product(idesc_k, next >= prm.ntiles);
             mma_commit(&bar_mma);
         }
-        if (!mbar_wait(&bar_mma, mma_phase)) ok = false;
+        __syncwarp();
+        if (!mbar_wait_warp(&bar_mma, mma_phase, lane)) ok = false;
         mma_phase ^= 1u;
         tc_fence_after();
         if (!__syncthreads_and(ok)) { ok = false; break; }
