@@ -1305,8 +1305,8 @@ size_t tc_request_bytes(int n, int N, int G)
     return std::max(tc_smem_bytes(n, N, G), floor_bytes);
 }
 
-// E too large for shared memory beside a tile (n > 224): the streamed tcgen05
-// form, 32 or 64 channels per tile, as many ring stages (up to 4) as fit.
+// E too large for shared memory beside a tile (n > 224) and tcgen05 asked for: the
+// streamed form, 32 or 64 channels per tile, as many ring stages (up to 4) as fit.
 msc_status setup_tc_stream(msc_plan *p, int sms, size_t optin)
 {
     const int n = p->n, kp = (n + 15) / 16 * 16, mt = (n + 127) / 128;
@@ -1362,7 +1362,11 @@ msc_status setup_tensor_core(msc_plan *p)
         chosen = N;
         if (tiles <= sms) break;   // enough tiles for every SM already at this width
     }
-    if (chosen == 0) return setup_tc_stream(p, sms, (size_t)optin);
+    // Above 224 nodes the inner solve keeps FP32 products unless the caller asks for
+    // tcgen05 (flag 2): against 64 bits a BF16x3 block inverse is 6.1e-6 to 7.0e-6 off
+    // (2-norm), the FP32 one 4.6e-7 to 4.8e-7, and on 4 x 81 x 81 x 300 over 32 inputs
+    // psi was up to 3 times as far off as with FP32 products (97 ms a solve, 49 with it).
+    if (chosen == 0) return (p->desc.flags & 2) ? setup_tc_stream(p, sms, (size_t)optin) : MSC_OK;
     p->tc_n = chosen;
     p->tc_groups = 1;
     p->tc_tile_rows = chosen / 2;

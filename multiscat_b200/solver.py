@@ -148,7 +148,8 @@ class ScatteringPlan:
         desc.inner_restart = inner_restart
         desc.inner_rtol = inner_rtol
         desc.max_refinements = max_refinements
-        # tensor_cores: None = autotuned, True = always tcgen05, False = never
+        # tensor_cores: None = autotuned up to 224 nodes and FP32 products above, True =
+        # always tcgen05 (BF16x3, up to 560 nodes), False = never
         desc.flags = {None: 0, True: 2, False: 1}[tensor_cores]
         # mixed form: Gram-Schmidt passes of the FP32 inner Arnoldi step (1 or 2)
         if inner_gram_schmidt_passes not in (1, 2):
