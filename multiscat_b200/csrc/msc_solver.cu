@@ -730,6 +730,7 @@ msc_status ensure_boxes(msc_plan *p, int kind)
         }
         MSC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::room));
         MSC_CUDA(upload(bx.work, wl));
+        MSC_CUDA(cudaStreamSynchronize(0));      // the autotuner launches on the plan's stream at once
         bx.nwork = (int)wl.size();
         bx.smem = smem;
         return MSC_OK;
