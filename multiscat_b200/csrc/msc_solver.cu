@@ -2178,6 +2178,7 @@ msc_status ensure_gs_levels(msc_plan *p)
                                   (int)smem_coupling(msc::kMaxTaps)));
     MSC_CUDA(cudaFuncSetAttribute(msc::k_coupling_masked<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)smem_coupling(msc::kMaxTaps)));
+    MSC_CUDA(cudaStreamSynchronize(0));      // the sweep may follow at once on any stream
     p->gs_ready = true;
     return MSC_OK;
 }

@@ -1,6 +1,6 @@
 // A stand-in for the CUDA runtime on a machine without a GPU: device memory is host
 // memory, copies and fills happen at once, kernels do nothing.  It records
-//  - launches on another stream while work of the legacy stream (allocations, copies,
+//  - launches, copies and fills on another stream while work of the legacy stream (allocations, copies,
 //    fills, kernels) may still be under way: no host wait and no event orders them
 //    (a copy to the device from pageable memory may return before it has arrived);
 //  - kernels in launch order, and fails the launches whose name holds FAKE_CUDA_FAIL.
@@ -32,10 +32,14 @@ cudaError_t set(cudaError_t e)
 }
 void touch(cudaStream_t s) { legacy += s == nullptr; }
 void join(cudaStream_t s) { if (!s) waited = legacy; }
+void check(cudaStream_t s, const std::string &what)
+{
+    if (s && !capturing && std::max(waited, stream_waited[s]) < legacy) report += "unordered " + what + "\n";
+}
 cudaError_t launch(const void *f, cudaStream_t s)
 {
     const std::string &n = names[f];
-    if (s && !capturing && std::max(waited, stream_waited[s]) < legacy) report += "unordered " + n + "\n";
+    check(s, n);
     report += "launch " + n + "\n";
     touch(s);
     const char *fail = std::getenv("FAKE_CUDA_FAIL");
@@ -105,11 +109,18 @@ cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind k)
 }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t st)
 {
+    check(st, "copy");
     std::memcpy(d, s, n);
     touch(st);
     return cudaSuccess;
 }
-cudaError_t cudaMemsetAsync(void *d, int v, size_t n, cudaStream_t s) { std::memset(d, v, n); touch(s); return cudaSuccess; }
+cudaError_t cudaMemsetAsync(void *d, int v, size_t n, cudaStream_t s)
+{
+    check(s, "fill");
+    std::memset(d, v, n);
+    touch(s);
+    return cudaSuccess;
+}
 
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { *s = static_cast<cudaStream_t>(handle()); return cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }

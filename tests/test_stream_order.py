@@ -23,3 +23,18 @@ assert any("k_coupling_box" in x for x in report("launch"))
 assert report("unordered") == [], report("unordered")
 lib.msc_plan_destroy(h)
 ''', tmp_path)
+
+
+@pytest.mark.parametrize("call", ["msc_solve_lower_block", "msc_apply_lower_block"])
+@pytest.mark.parametrize("solved_before", [False, True])
+def test_lower_block_waits_for_its_tables(call, solved_before, tmp_path):
+    # on a plan that was not made for Gauss-Seidel: the level tables are built by this call
+    fake_cuda.run(f'''
+h = plan(30, 9, separable=False)
+res = nat.Result()
+if {solved_before}:
+    lib.msc_solve(h, None, None, ctypes.byref(res), side)
+assert lib.{call}(h, buf(h), buf(h), side) == 0
+assert report("unordered") == [], report("unordered")
+lib.msc_plan_destroy(h)
+''', tmp_path)
