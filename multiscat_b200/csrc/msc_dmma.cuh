@@ -147,6 +147,14 @@ __host__ __device__ constexpr size_t smem_bytes(int n, int cl)
     return (cols * col_stride(n) + tr + 2 * tr * (kWM + cl + 1) + 2 * 32 * 8) * sizeof(double);
 }
 
+// The two halves of a cluster barrier; the arrival orders no memory, it only says that
+// the CTA has started.
+__device__ __forceinline__ void cluster_arrive()
+{
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
+
 // Any system of rows [row0, row0 + nrow) still active?  (same answer in every thread)
 __device__ __forceinline__ bool tile_active(const Params &p, int row0, int nrow)
 {
@@ -207,6 +215,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_block_inverse_dmma(Params p)
     const int row0 = (int)(blockIdx.x / cl) * TR;
     const int nrow = min(TR, p.rows - row0);
     if (!tile_active(p, row0, nrow)) return;                     // same for the whole cluster
+    // Shared memory of another CTA may be touched once that CTA runs: the arrival is
+    // waited for where the sums are sent, behind the first product.
+    if (cl > 1) cluster_arrive();
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wm = warp & (kWM - 1), wn = warp >> 2;
@@ -256,6 +267,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_block_inverse_dmma(Params p)
     }
     __syncthreads();
     if (cl > 1) {
+        cluster_wait();        // every CTA of the cluster has started
         for (int t = threadIdx.x; t < cl * TR; t += kThreads) {
             const int dst = t / TR, r = t - dst * TR;
             double2 v = sred[r];
