@@ -262,9 +262,12 @@ k_apply_rotations(int n, int ngroups, int nsteps, const int4 *__restrict__ group
     extern __shared__ __align__(16) double zs_all[];
     double2 *ring = reinterpret_cast<double2 *>(zs_all);      // [3][kRotChunk][4]
     double *zs = zs_all + (size_t)3 * kRotChunk * 8;          // [n][RB]
-    const int t = threadIdx.x % RB;                           // (RB = 16: lanes 16.. shadow 0..15)
+    const int t = threadIdx.x % RB;                           // (RB = 16: lanes 16.. read as 0..15, write nothing)
     const int row = blockIdx.x * RB + t;
-    for (int c = 0; c < n; ++c) zs[c * RB + t] = (c == row) ? 1.0 : 0.0;
+    const bool own = threadIdx.x < RB;                        // one lane writes a cell
+    if (own)
+        for (int c = 0; c < n; ++c) zs[c * RB + t] = (c == row) ? 1.0 : 0.0;
+    __syncwarp();
     // chunk q of the table into ring slot q % 3; past the end nothing is copied
     auto fetch = [&](int q) {
         const int lo = q * kRotChunk * 4, hi = min(nsteps, (q + 1) * kRotChunk) * 4;
@@ -303,7 +306,7 @@ k_apply_rotations(int n, int ngroups, int nsteps, const int4 *__restrict__ group
                 on[j] = fma(r.x, carry[j], r.y * qb);
                 carry[j] = fma(-r.y, carry[j], r.x * qb);
             }
-            if (!EDGE || st >= 6) zs[(lo + st - 6) * RB + t] = on[3];
+            if (own && (!EDGE || st >= 6)) zs[(lo + st - 6) * RB + t] = on[3];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 if (EDGE) o2[j] = o1[j];
@@ -312,7 +315,9 @@ k_apply_rotations(int n, int ngroups, int nsteps, const int4 *__restrict__ group
         };
         for (int st = 0; st < L + 6;) {
             if (pos % kRotChunk == 0) {
-                // the next chunk but one is requested while this one is used
+                // the next chunk but one is requested while this one is used, into the slot
+                // of the chunk before it, which every lane has to be done with
+                __syncwarp();
                 fetch(pos / kRotChunk + 2);
                 asm volatile("cp.async.wait_group 2;" ::: "memory");
                 __syncwarp();
@@ -326,11 +331,11 @@ k_apply_rotations(int n, int ngroups, int nsteps, const int4 *__restrict__ group
             for (; st < end; ++st, cs += 4) step(st, cs, std::true_type{});
             pos += run;
         }
-        zs[(lo + L) * RB + t] = carry[3];
+        if (own) zs[(lo + L) * RB + t] = carry[3];
         gr = gnext;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    if (row < n && threadIdx.x < RB)
+    if (row < n && own)
         for (int c = 0; c < n; ++c) Zt[(size_t)c * n + row] = zs[c * RB + t];
 }
 
