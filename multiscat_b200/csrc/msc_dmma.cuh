@@ -427,7 +427,7 @@ cudaError_t instance(bool inverse, const Config &c, const Params &p, cudaStream_
     const int tiles = (p.rows + 8 * NTW - 1) / (8 * NTW);
     if (!inverse) {
         res<<<dim3(tiles, c.cl), kThreads, smem_for(NTW, p.n, 1), st>>>(p);
-        return cudaGetLastError();
+        return cudaPeekAtLastError();       // (the caller's own check still sees it)
     }
     cudaLaunchConfig_t lc{};
     lc.gridDim = dim3(tiles * c.cl);

@@ -355,6 +355,7 @@ struct msc_plan {
     int fallbacks_last = 0;              // systems re-solved in FP64 by the last msc_solve
     int64_t launches_cycle = 0;          // kernel nodes of the cycle graph
     int solves = 0;                      // msc_solve calls so far
+    cudaError_t launch_error = cudaSuccess;   // first failed launch since the last check
 
     ~msc_plan()
     {
@@ -391,6 +392,28 @@ struct msc_plan {
 };
 
 namespace {
+
+// A failed launch, kept until launched() reports it: a missing kernel instance leaves no
+// error in the runtime.
+void note_launch(msc_plan *p, cudaError_t e)
+{
+    if (e != cudaSuccess && p->launch_error == cudaSuccess) p->launch_error = e;
+}
+
+// Whether every launch of the plan since the last check succeeded.
+msc_status launched(msc_plan *p)
+{
+    const cudaError_t last = cudaGetLastError(), e = p->launch_error != cudaSuccess ? p->launch_error : last;
+    p->launch_error = cudaSuccess;
+    if (e != cudaSuccess) return fail(MSC_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
+    return MSC_OK;
+}
+
+#define MSC_LAUNCHED(plan)                                   \
+    do {                                                     \
+        const msc_status launched_ = launched(plan);         \
+        if (launched_ != MSC_OK) return launched_;           \
+    } while (0)
 
 template <typename T>
 cudaError_t upload(DevBuf<T> &buf, const std::vector<T> &h)
@@ -466,7 +489,7 @@ cudaError_t tcs_instance(const msc::tc::TcStreamParams &sp, int grid, cudaStream
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
     msc::tc::k_block_inverse_tcs<N, S>
         <<<grid, msc::tc::kThreads, msc::tc::stream_smem(sp.t.kp, N, S), st>>>(sp);
-    return cudaGetLastError();
+    return cudaPeekAtLastError();
 }
 
 cudaError_t tcs_dispatch(int N, int S, const msc::tc::TcStreamParams &sp, int grid, cudaStream_t st, int limit)
@@ -505,7 +528,7 @@ void launch_block_inverse_tc(msc_plan *p, const int *gate, const float2 *x, floa
     constexpr int T = msc::tc::kThreads;
     if (p->tc_groups == kTcStream) {
         const msc::tc::TcStreamParams sp{prm, p->e_img_zk.p, p->e_img_kz.p};
-        (void)tcs_dispatch(p->tc_n, p->tcs_stages[p->tc_n == 128], sp, p->tc_grid, st, 0);
+        note_launch(p, tcs_dispatch(p->tc_n, p->tcs_stages[p->tc_n == 128], sp, p->tc_grid, st, 0));
         return;
     }
     if (p->tc_groups == kTcChannelMajor) {
@@ -560,7 +583,7 @@ void launch_block_inverse(msc_plan *p, const int *gate, const double2 *x, double
     msc::dm::Params q = dmma_params(p, gate, x, out, acc);
     q.img1 = p->img_et.p;
     q.img2 = p->img_e.p;
-    (void)msc::dm::dispatch(true, msc::dm::choose(p->R, p->n), q, st, true);
+    note_launch(p, msc::dm::dispatch(true, msc::dm::choose(p->R, p->n), q, st, true));
 }
 
 template <typename R>
@@ -591,7 +614,7 @@ void launch_residual_diag(msc_plan *p, const int *gate, const double2 *x, double
 {
     msc::dm::Params q = dmma_params(p, gate, x, out, with_b);
     q.img1 = p->img_t.p;
-    (void)msc::dm::dispatch(false, msc::dm::choose(p->R, p->n), q, st, true);
+    note_launch(p, msc::dm::dispatch(false, msc::dm::choose(p->R, p->n), q, st, true));
 }
 
 // The halo kernel instance of (window reach, outputs per thread, precision, mask) as a
@@ -1165,6 +1188,11 @@ msc_status capture(msc_plan *p, void (*rec)(msc_plan *, cudaStream_t), cudaGraph
         rec(p, p->stream);
         e = cudaStreamEndCapture(p->stream, &graph);
     }
+    const msc_status recorded = launched(p);     // a launch that failed is missing from the graph
+    if (recorded != MSC_OK) {
+        if (e == cudaSuccess) cudaGraphDestroy(graph);
+        return recorded;
+    }
     if (e != cudaSuccess) return fail(MSC_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
     if (kernel_nodes) *kernel_nodes = count_kernel_nodes(graph);
     e = cudaGraphInstantiate(out, graph, 0);
@@ -1636,7 +1664,7 @@ msc_status autotune_measure(msc_plan *p)
             }
         }
     }
-    MSC_CUDA(cudaGetLastError());
+    MSC_LAUNCHED(p);
     return MSC_OK;
 }
 
@@ -2715,7 +2743,7 @@ msc_status msc_solve(msc_plan *p, double *psi_out, double *intensities_out, msc_
     const int max_cycles = p->desc.max_iterations + 2;
     const bool x_zero = !p->has_x0;
     record_cycle_start_t(p, x_zero, ps);
-    MSC_CUDA(cudaGetLastError());
+    MSC_LAUNCHED(p);
     int64_t launches = 1 + cycle_start_launches(x_zero);
     bool live = true;
     if (!x_zero) {
@@ -2740,7 +2768,7 @@ msc_status msc_solve(msc_plan *p, double *psi_out, double *intensities_out, msc_
             MSC_CUDA(cudaGraphLaunch(p->g_cycle, ps));
         } else {
             record_cycle(p, ps);
-            MSC_CUDA(cudaGetLastError());
+            MSC_LAUNCHED(p);
         }
         launches += p->g_cycle ? p->launches_cycle : cycle_launches(p);
         MSC_CUDA(cudaStreamSynchronize(ps));
@@ -2758,13 +2786,13 @@ msc_status msc_solve(msc_plan *p, double *psi_out, double *intensities_out, msc_
             msc::k_intensities<<<(p->R + 255) / 256, 256, 0, ps>>>(
                 p->R, 0, p->n, p->row_sys.p, p->sys_spec_row.p, p->sys_aspec.p, p->row_b.p, p->X.p,
                 intensities_out);
-            MSC_CUDA(cudaGetLastError());
+            MSC_LAUNCHED(p);
         }
         return MSC_OK;
     };
     msc::k_solve_report<<<sys_blocks(p->B + 1), 128, 0, ps>>>(p->state(), p->B, p->use_tc ? p->tc_error.p : nullptr,
                                                               p->wait_error.p, p->report.p);
-    MSC_CUDA(cudaGetLastError());
+    MSC_LAUNCHED(p);
     MSC_CUDA(cudaMemcpyAsync(p->report_host, p->report.p, (size_t)(p->B + 1) * sizeof(msc::SolveReport),
                              cudaMemcpyDeviceToHost, ps));
     st = write_outputs();
@@ -2881,7 +2909,7 @@ msc_status msc_debug_apply_coupling(msc_plan *p, const double *x, double *y, voi
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     launch_coupling(p, nullptr, reinterpret_cast<const double2 *>(x), nullptr, 1.0,
                     reinterpret_cast<double2 *>(y), s);
-    MSC_CUDA(cudaGetLastError());
+    MSC_LAUNCHED(p);
     return MSC_OK;
 }
 
@@ -2893,7 +2921,7 @@ msc_status msc_debug_apply_block_inverse(msc_plan *p, const double *x, double *y
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     launch_block_inverse(p, nullptr, reinterpret_cast<const double2 *>(x),
                          reinterpret_cast<double2 *>(y), 0, s);
-    MSC_CUDA(cudaGetLastError());
+    MSC_LAUNCHED(p);
     return MSC_OK;
 }
 
@@ -2911,7 +2939,7 @@ msc_status msc_debug_apply_operator(msc_plan *p, const double *x, double *y, voi
     const size_t cnt = (size_t)p->R * p->n;
     msc::k_scale<<<(unsigned)std::min<size_t>((cnt + 255) / 256, 4096), 256, 0, s>>>(
         reinterpret_cast<double2 *>(y), cnt, -1.0);
-    MSC_CUDA(cudaGetLastError());
+    MSC_LAUNCHED(p);
     return MSC_OK;
 }
 
@@ -2931,7 +2959,7 @@ msc_status msc_apply_lower_block(msc_plan *p, const double *x, double *y, void *
     const size_t cnt = (size_t)p->R * p->n;
     msc::k_scale<<<(unsigned)std::min<size_t>((cnt + 255) / 256, 4096), 256, 0, s>>>(
         reinterpret_cast<double2 *>(y), cnt, -1.0);
-    MSC_CUDA(cudaGetLastError());
+    MSC_LAUNCHED(p);
     return MSC_OK;
 }
 
@@ -2945,7 +2973,7 @@ msc_status msc_solve_lower_block(msc_plan *p, const double *x, double *y, void *
     if (st != MSC_OK) return st;
     launch_gs_sweep_t<double>(p, nullptr, reinterpret_cast<const double2 *>(x),
                               reinterpret_cast<double2 *>(y), reinterpret_cast<cudaStream_t>(stream));
-    MSC_CUDA(cudaGetLastError());
+    MSC_LAUNCHED(p);
     return MSC_OK;
 }
 
@@ -2983,7 +3011,7 @@ msc_status msc_debug_apply_block_inverse_f32(msc_plan *p, const float *x, float 
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     launch_block_inverse_t<float>(p, nullptr, reinterpret_cast<const float2 *>(x),
                                   reinterpret_cast<float2 *>(y), 0, s);
-    MSC_CUDA(cudaGetLastError());
+    MSC_LAUNCHED(p);
     if (p->use_tc) {
         int tc_err = 0;
         MSC_CUDA(cudaMemcpyAsync(&tc_err, p->tc_error.p, sizeof(int), cudaMemcpyDeviceToHost, s));
