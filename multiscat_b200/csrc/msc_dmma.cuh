@@ -479,13 +479,16 @@ inline cudaError_t set_attributes()
 // CTAs' column buffers fit in one SM; and for few rows narrow tiles with the
 // M rows split further while every CTA still has an SM to itself and more
 // than one m-tile per warp.  784 us is 74% of the DMMA rate.
-inline Config choose(int rows, int n)
+// The residual (one product, x staged by every M slice) takes the same split; measured,
+// us at it / at its own best: 121 x 100 5.1 / 5.1, 100 x 550 17.0 / 17.0, 1681 x 200 21.1 /
+// 19.5 (3/4), 26244 x 300 386 / 386, 29856 x 150 140 / 137 (2/1), 119409 x 150 461 / 461.
+inline Config choose(int rows, int n, int sms)
 {
     int cl = 1;
     while (mt_of(n, cl) > 5) cl *= 2;
     const int narrow = (rows + 7) / 8;
-    if (narrow * cl <= 2 * 148) {
-        while (cl < 8 && 2 * cl * narrow <= 148 && mt_of(n, cl) > 1) cl *= 2;
+    if (narrow * cl <= 2 * sms) {
+        while (cl < 8 && 2 * cl * narrow <= sms && mt_of(n, cl) > 1) cl *= 2;
         return Config{1, cl, mt_of(n, cl)};
     }
     const int ntw = 2 * (smem_for(3, n, cl) + 1024) <= 228 * 1024 ? 3

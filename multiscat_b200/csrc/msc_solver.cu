@@ -253,6 +253,7 @@ struct msc_plan {
     std::vector<SystemHost> sys;
     // rows / tiles
     int R = 0, ntiles = 0;
+    int sms = 0;                   // SMs of the plan's device
     std::vector<int> tile_row0_h, tile_nrow_h, tile_sys_h, sys_tile0_h, sys_row0_h, row_sys_h;
     // device data
     DevBuf<double> E, Tm, lam, en, v00, row_pkd, row_fn;
@@ -583,7 +584,7 @@ void launch_block_inverse(msc_plan *p, const int *gate, const double2 *x, double
     msc::dm::Params q = dmma_params(p, gate, x, out, acc);
     q.img1 = p->img_et.p;
     q.img2 = p->img_e.p;
-    note_launch(p, msc::dm::dispatch(true, msc::dm::choose(p->R, p->n), q, st, true));
+    note_launch(p, msc::dm::dispatch(true, msc::dm::choose(p->R, p->n, p->sms), q, st, true));
 }
 
 template <typename R>
@@ -614,7 +615,7 @@ void launch_residual_diag(msc_plan *p, const int *gate, const double2 *x, double
 {
     msc::dm::Params q = dmma_params(p, gate, x, out, with_b);
     q.img1 = p->img_t.p;
-    note_launch(p, msc::dm::dispatch(false, msc::dm::choose(p->R, p->n), q, st, true));
+    note_launch(p, msc::dm::dispatch(false, msc::dm::choose(p->R, p->n, p->sms), q, st, true));
 }
 
 // The halo kernel instance of (window reach, outputs per thread, precision, mask) as a
@@ -1490,9 +1491,7 @@ msc_status autotune_measure(msc_plan *p);
 
 void apply_tc_width(msc_plan *p, int N, int G = 1)
 {
-    int sms = 148, dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = p->sms;
     if (p->tc_groups == kTcStream) {           // n > 224: the only form that fits
         p->tc_n = N >= 128 && p->tcs_stages[1] ? 128 : p->tcs_stages[0] ? 64 : 128;
         p->tc_tile_rows = p->tc_n / 2;
@@ -1952,7 +1951,7 @@ msc_status finalize(msc_plan *p)
                 p->halo_by = bh;
                 p->halo_seg = seg;
                 const int lines = (n + msc::halo_zc<double>() - 1) / msc::halo_zc<double>();
-                if ((int64_t)wl.size() * lines >= 3 * 148 && bh > msc::kHaloMax) break;
+                if ((int64_t)wl.size() * lines >= 3 * p->sms && bh > msc::kHaloMax) break;
             }
             p->nwork = (int)wl.size();
             MSC_CUDA(upload(p->tap_window, win));
@@ -2015,8 +2014,8 @@ msc_status finalize(msc_plan *p)
             for (int s = 0; s < p->B; ++s) k += (p->sys[s].C + rows - 1) / rows;
             return k;
         };
-        int crow = std::min(crow_max, std::max(1, p->R / (2 * 148)));
-        while (crow < crow_max && blocks_at(crow) > 2 * 148) ++crow;
+        int crow = std::min(crow_max, std::max(1, p->R / (2 * p->sms)));
+        while (crow < crow_max && blocks_at(crow) > 2 * p->sms) ++crow;
         std::vector<int> c0, cn, cs, sc0(p->B + 1);
         for (int s = 0; s < p->B; ++s) {
             sc0[s] = (int)c0.size();
@@ -2032,7 +2031,7 @@ msc_status finalize(msc_plan *p)
         }
         sc0[p->B] = (int)c0.size();
         p->nchunks = (int)c0.size();
-        p->chunk_short = p->nchunks <= 2 * 148 && crow * n <= 2048;
+        p->chunk_short = p->nchunks <= 2 * p->sms && crow * n <= 2048;
         // the streamed reduction takes chunks of at most kBulkChunk elements
         // on 16-byte boundaries (n even: every chunk starts on an even element)
         const int max_rows = cn.empty() ? 0 : *std::max_element(cn.begin(), cn.end());
@@ -2505,9 +2504,12 @@ msc_status msc_plan_create(msc_plan **plan, const msc_plan_desc *desc)
     p->sys.resize(p->B);
     msc_status st = set_kernel_attributes();
     if (st != MSC_OK) { delete p; return st; }
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, dev);
     // pinned block: the counter, the results and the cycle's step counts
     const size_t o_report = 64, o_kcyc = o_report + (size_t)(p->B + 1) * sizeof(msc::SolveReport);
-    cudaError_t e = kit_acquire(o_kcyc + (size_t)p->B * sizeof(int), &p->kit);
+    if (e == cudaSuccess) e = kit_acquire(o_kcyc + (size_t)p->B * sizeof(int), &p->kit);
     if (e != cudaSuccess) {
         delete p;
         return fail(MSC_ERR_CUDA, std::string("plan create: ") + cudaGetErrorString(e));
@@ -3170,7 +3172,7 @@ msc_status msc_potential_gradient(msc_plan *p, const double *psi, const double *
         const int ndyb = (wy + kd - 1) / kd;
         const int dx_max = std::max(1, 256 / ndyb);
         if (ndyb <= 256) {
-            const int want = std::max((wx + dx_max - 1) / dx_max, std::min(wx, (4 * 148 + n - 1) / n));
+            const int want = std::max((wx + dx_max - 1) / dx_max, std::min(wx, (4 * p->sms + n - 1) / n));
             const int dxc = (wx + want - 1) / want;
             const dim3 g((wx + dxc - 1) / dxc, n);
             const int nt = (dxc * ndyb + 31) / 32 * 32;

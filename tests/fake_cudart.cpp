@@ -4,7 +4,8 @@
 //    fills, kernels) may still be under way: no host wait and no event orders them
 //    (a copy to the device from pageable memory may return before it has arrived);
 //  - kernels in launch order, and fails the launches whose name holds FAKE_CUDA_FAIL.
-// fake_report() returns one line per event: "unordered NAME" or "launch NAME".
+// fake_report() returns one line per event: "unordered NAME", "launch NAME" or "grid X Y NAME".
+// FAKE_CUDA_SMS: the device's SM count (148).
 #include <cuda_runtime_api.h>
 
 #include <cstdlib>
@@ -36,11 +37,11 @@ void check(cudaStream_t s, const std::string &what)
 {
     if (s && !capturing && std::max(waited, stream_waited[s]) < legacy) report += "unordered " + what + "\n";
 }
-cudaError_t launch(const void *f, cudaStream_t s)
+cudaError_t launch(const void *f, dim3 grid, cudaStream_t s)
 {
     const std::string &n = names[f];
     check(s, n);
-    report += "launch " + n + "\n";
+    report += "launch " + n + "\ngrid " + std::to_string(grid.x) + " " + std::to_string(grid.y) + " " + n + "\n";
     touch(s);
     const char *fail = std::getenv("FAKE_CUDA_FAIL");
     return set(fail && *fail && n.find(fail) != std::string::npos ? cudaErrorInvalidConfiguration : cudaSuccess);
@@ -67,8 +68,8 @@ cudaError_t __cudaPopCallConfiguration(dim3 *g, dim3 *b, size_t *m, void *s)
     *g = cfg_grid; *b = cfg_block; *m = cfg_smem; *static_cast<cudaStream_t *>(s) = cfg_stream;
     return cudaSuccess;
 }
-cudaError_t cudaLaunchKernel(const void *f, dim3, dim3, void **, size_t, cudaStream_t s) { return launch(f, s); }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **) { return launch(f, c->stream); }
+cudaError_t cudaLaunchKernel(const void *f, dim3 g, dim3, void **, size_t, cudaStream_t s) { return launch(f, g, s); }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **) { return launch(f, c->gridDim, c->stream); }
 
 cudaError_t cudaGetLastError() { cudaError_t e = last; last = cudaSuccess; return e; }
 cudaError_t cudaPeekAtLastError() { return last; }
@@ -77,7 +78,8 @@ const char *cudaGetErrorString(cudaError_t) { return "fake error"; }
 cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr a, int)
 {
-    *v = a == cudaDevAttrMultiProcessorCount ? 148 : a == cudaDevAttrComputeCapabilityMajor ? 10
+    const char *sms = std::getenv("FAKE_CUDA_SMS");
+    *v = a == cudaDevAttrMultiProcessorCount ? (sms ? std::atoi(sms) : 148) : a == cudaDevAttrComputeCapabilityMajor ? 10
          : a == cudaDevAttrComputeCapabilityMinor ? 0 : a == cudaDevAttrMaxSharedMemoryPerBlockOptin ? 232448 : 0;
     return cudaSuccess;
 }
