@@ -1524,7 +1524,8 @@ void apply_tc_width(msc_plan *p, int N, int G = 1)
 // MSC_TUNE="c64=K,c32=K,bi=N[,bg=G]" fixes the choices (K: 0 neighbour
 // table, 1 / 2 halo tiles with one / two threads per patch column, 3 to 5 separable
 // over channel boxes; N: tcgen05 tile width,
-// 0 = SIMT; G: 1 or 2 warp groups in the tcgen05 kernel, default 1).
+// 0 = SIMT; G: 1 or 2 warp groups in the tcgen05 kernel, 3 the channel-major kernel,
+// default 1; above 224 nodes N picks the width of the streamed kernel).
 // Profiling runs use it so that a profiler's overhead cannot change what the
 // autotuner picks.
 bool tune_from_env(msc_plan *p)

@@ -53,9 +53,7 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void *src, uint32_t bytes
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 
-// Largest kp (what the shared memory takes), and the units of 8 accumulator columns
-// that a warp reads from TMEM at a time.
-constexpr int kTccMaxKp = 176, kTccBatch = 1;
+constexpr int kTccMaxKp = 176;      // largest kp: what the shared memory takes
 
 // One CTA per SM, 512 threads: warp w reads TMEM lanes 32 (w % 4) .. + 31
 // (rows c, i.e. 16 channels) and the column group w / 4 (a quarter of kp,
@@ -313,23 +311,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tcc(TcParams prm)
             // not as a tree, and near a resonance of H0 + pkd they cancel)
             double sacc = 0.0;
 #pragma unroll 1
-            for (int ub = 0; ub < nu; ub += kTccBatch) {
-                uint32_t r[kTccBatch][8], w[kTccBatch][8];
-#pragma unroll
-                for (int q = 0; q < kTccBatch; ++q)
-                    if (ub + q < nu) {
-                        tmem_ld8_nowait(t1 + (uint32_t)(8 * (ub + q)), r[q]);
-                        tmem_ld8_nowait(t2 + (uint32_t)(8 * (ub + q)), w[q]);
-                    }
+            for (int u = 0; u < nu; ++u) {
+                uint32_t r[8], w[8];
+                tmem_ld8_nowait(t1 + (uint32_t)(8 * u), r);
+                tmem_ld8_nowait(t2 + (uint32_t)(8 * u), w);
                 tmem_wait_ld();
 #pragma unroll
-                for (int q = 0; q < kTccBatch; ++q) {
-                    if (ub + q >= nu) continue;
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        const float we = en_s[8 * (u0 + ub + q) + e] * __uint_as_float(w[q][e]);
-                        sacc = fma((double)we, (double)__uint_as_float(r[q][e]), sacc);
-                    }
+                for (int e = 0; e < 8; ++e) {
+                    const float we = en_s[8 * (u0 + u) + e] * __uint_as_float(w[e]);
+                    sacc = fma((double)we, (double)__uint_as_float(r[e]), sacc);
                 }
             }
             sm_part[cg][c] = sacc;
@@ -349,34 +339,26 @@ __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tcc(TcParams prm)
             const double2 b = cmul(cf_s[jc], make_double2(sr, si));
             const float bpart = (float)(part ? b.y : b.x);
 #pragma unroll 1
-            for (int ub = 0; ub < nu; ub += kTccBatch) {
-                uint32_t r[kTccBatch][8], w[kTccBatch][8];
-#pragma unroll
-                for (int q = 0; q < kTccBatch; ++q)
-                    if (ub + q < nu) {
-                        tmem_ld8_nowait(t1 + (uint32_t)(8 * (ub + q)), r[q]);
-                        tmem_ld8_nowait(t2 + (uint32_t)(8 * (ub + q)), w[q]);
-                    }
+            for (int u = 0; u < nu; ++u) {
+                uint32_t r[8], w[8];
+                tmem_ld8_nowait(t1 + (uint32_t)(8 * u), r);
+                tmem_ld8_nowait(t2 + (uint32_t)(8 * u), w);
                 tmem_wait_ld();
+                const int k0 = 8 * (u0 + u);
+                uint32_t hw[4], lw[4];
 #pragma unroll
-                for (int q = 0; q < kTccBatch; ++q) {
-                    if (ub + q >= nu) continue;
-                    const int k0 = 8 * (u0 + ub + q);
-                    uint32_t hw[4], lw[4];
-#pragma unroll
-                    for (int e = 0; e < 8; e += 2) {
-                        const float y0 = (__uint_as_float(r[q][e]) + bpart * en_s[k0 + e]) * __uint_as_float(w[q][e]);
-                        const float y1 = (__uint_as_float(r[q][e + 1]) + bpart * en_s[k0 + e + 1]) * __uint_as_float(w[q][e + 1]);
-                        const __nv_bfloat162 h = __floats2bfloat162_rn(y0, y1);
-                        const float2 fh = __bfloat1622float2(h);
-                        const __nv_bfloat162 l = __floats2bfloat162_rn(y0 - fh.x, y1 - fh.y);
-                        hw[e >> 1] = *reinterpret_cast<const uint32_t *>(&h);
-                        lw[e >> 1] = *reinterpret_cast<const uint32_t *>(&l);
-                    }
-                    const uint32_t o = kmaj_off(c, k0, ROWS);
-                    *reinterpret_cast<uint4 *>(a_hi + o) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-                    *reinterpret_cast<uint4 *>(a_lo + o) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+                for (int e = 0; e < 8; e += 2) {
+                    const float y0 = (__uint_as_float(r[e]) + bpart * en_s[k0 + e]) * __uint_as_float(w[e]);
+                    const float y1 = (__uint_as_float(r[e + 1]) + bpart * en_s[k0 + e + 1]) * __uint_as_float(w[e + 1]);
+                    const __nv_bfloat162 h = __floats2bfloat162_rn(y0, y1);
+                    const float2 fh = __bfloat1622float2(h);
+                    const __nv_bfloat162 l = __floats2bfloat162_rn(y0 - fh.x, y1 - fh.y);
+                    hw[e >> 1] = *reinterpret_cast<const uint32_t *>(&h);
+                    lw[e >> 1] = *reinterpret_cast<const uint32_t *>(&l);
                 }
+                const uint32_t o = kmaj_off(c, k0, ROWS);
+                *reinterpret_cast<uint4 *>(a_hi + o) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+                *reinterpret_cast<uint4 *>(a_lo + o) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
             }
         }
         tc_fence_before();
@@ -417,35 +399,29 @@ __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tcc(TcParams prm)
         // whole values of a unit.)
         float2 *urow = raw + (size_t)jc * n;
 #pragma unroll 1
-        for (int ub = 0; ub < nu; ub += kTccBatch) {
-            uint32_t r[kTccBatch][8];
-#pragma unroll
-            for (int q = 0; q < kTccBatch; ++q)
-                if (ub + q < nu) tmem_ld8_nowait(t2 + (uint32_t)(8 * (ub + q)), r[q]);
+        for (int u = 0; u < nu; ++u) {
+            uint32_t r[8];
+            tmem_ld8_nowait(t2 + (uint32_t)(8 * u), r);
             tmem_wait_ld();
+            const int z = 8 * (u0 + u) + 4 * part;
+            float2 o[4];
 #pragma unroll
-            for (int q = 0; q < kTccBatch; ++q) {
-                if (ub + q >= nu) continue;
-                const int z = 8 * (u0 + ub + q) + 4 * part;
-                float2 o[4];
+            for (int i = 0; i < 4; ++i) {
+                const float a = __uint_as_float(r[i]), b = __uint_as_float(r[4 + i]);
+                const float recv = __shfl_xor_sync(0xffffffffu, part ? a : b, 1);
+                o[i] = part ? make_float2(recv, b) : make_float2(a, recv);
+            }
+            if (!row_ok) continue;
+            if ((n & 1) == 0) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float a = __uint_as_float(r[q][i]), b = __uint_as_float(r[q][4 + i]);
-                    const float recv = __shfl_xor_sync(0xffffffffu, part ? a : b, 1);
-                    o[i] = part ? make_float2(recv, b) : make_float2(a, recv);
-                }
-                if (!row_ok) continue;
-                if ((n & 1) == 0) {
+                for (int i = 0; i < 4; i += 2)
+                    if (z + i < n)
+                        *reinterpret_cast<float4 *>(urow + z + i) =
+                            make_float4(o[i].x, o[i].y, o[i + 1].x, o[i + 1].y);
+            } else {
 #pragma unroll
-                    for (int i = 0; i < 4; i += 2)
-                        if (z + i < n)
-                            *reinterpret_cast<float4 *>(urow + z + i) =
-                                make_float4(o[i].x, o[i].y, o[i + 1].x, o[i + 1].y);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        if (z + i < n) urow[z + i] = o[i];
-                }
+                for (int i = 0; i < 4; ++i)
+                    if (z + i < n) urow[z + i] = o[i];
             }
         }
         tc_fence_before();
