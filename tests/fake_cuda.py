@@ -1,20 +1,25 @@
 """The native library on a recorded stand-in for the CUDA runtime (fake_cudart.cpp).
 
-``run(script, tmp_path)`` compiles the stand-in, preloads it in a child process and
+``run(script)`` compiles the stand-in once, preloads it in a child process and
 runs ``script`` there after a prelude that loads the library and gives
 
 - ``nat``, ``lib``: the ctypes binding and the library (no torch in this process);
-- ``plan(n, torus, separable, mixed, flags)``: a finished plan handle, not yet solved;
+- ``plan(n, torus, separable, mixed, flags, reach)``: a plan of one full-torus system with
+  taps up to ``reach``, not yet solved;
 - ``side``: a caller's stream handle; ``buf(plan)``: a device vector of the plan;
-- ``report(prefix)``: the recorded names that follow ``prefix`` (\"unordered\", \"launch\").
+- ``report(prefix)``: the recorded names that follow ``prefix`` ("unordered", "launch").
 """
 
 from __future__ import annotations
 
+import atexit
+import functools
 import os
 import pathlib
+import shutil
 import subprocess
 import sys
+import tempfile
 
 from multiscat_b200 import build
 
@@ -38,14 +43,14 @@ def report(prefix):
     lines = fake.fake_report().decode().splitlines()
     return [x.split(" ", 1)[1] for x in lines if x.startswith(prefix + " ")]
 
-def plan(n, torus, separable, mixed=False, flags=0):
+def plan(n, torus, separable, mixed=False, flags=0, reach=1):
     rng = np.random.default_rng(n)
     d = nat.PlanDesc()
     d.n_z, d.nkx, d.nky, d.n_systems = n, torus, torus, 1
     d.restart, d.max_iterations, d.rtol, d.precision, d.flags = 30, 100, 1e-10, int(mixed), flags
     v = np.zeros((torus, torus, n), complex)
-    k = np.arange(-1, 2)
-    f = rng.uniform(0.5, 1.0, (3, 3))
+    k = np.arange(-reach, reach + 1)
+    f = rng.uniform(0.5, 1.0, (k.size, k.size))
     if separable:
         f = np.outer(f[0], f[1])
     v[np.ix_(k % torus, k % torus)] = f[:, :, None] * rng.uniform(0.5, 1.0, n)
@@ -68,15 +73,20 @@ def buf(h):
 '''
 
 
-def run(script: str, tmp_path, **env) -> str:
-    so = tmp_path / "libfake_cudart.so"
-    if not so.exists():
-        include = pathlib.Path(build.nvcc_path()).resolve().parent.parent / "include"
-        subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", f"-I{include}", str(HERE / "fake_cudart.cpp"),
-                        "-o", str(so)], check=True)
-    full = {**os.environ, "LD_PRELOAD": str(so), **env}
-    full.pop("MSC_TUNE", None)
-    full.update({k: v for k, v in env.items() if k == "MSC_TUNE"})
+@functools.cache
+def stand_in() -> str:
+    folder = tempfile.mkdtemp(prefix="fake_cudart_")
+    atexit.register(shutil.rmtree, folder, ignore_errors=True)
+    so = pathlib.Path(folder) / "libfake_cudart.so"
+    include = pathlib.Path(build.nvcc_path()).resolve().parent.parent / "include"
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", f"-I{include}", str(HERE / "fake_cudart.cpp"),
+                    "-o", str(so)], check=True)
+    return str(so)
+
+
+def run(script: str, **env) -> str:
+    full = {k: v for k, v in os.environ.items() if k != "MSC_TUNE"}
+    full.update(env, LD_PRELOAD=stand_in())
     p = subprocess.run([sys.executable, "-c", PRELUDE + script, str(HERE.parent / "multiscat_b200" / "_native.py")],
                        env=full, capture_output=True, text=True, timeout=300)
     assert p.returncode == 0, p.stdout + p.stderr

@@ -25,7 +25,7 @@ CALLS = {
 
 
 @pytest.mark.parametrize("kernel,made", CASES)
-def test_a_failed_launch_is_an_error(kernel, made, tmp_path):
+def test_a_failed_launch_is_an_error(kernel, made):
     # MSC_TUNE: the streamed form stays chosen, nothing is measured
     fake_cuda.run(f'''
 h = {made}
@@ -38,14 +38,14 @@ h = {made}
 st = {CALLS.get(kernel, "nat.MSC_ERR_CUDA")}
 assert st == nat.MSC_ERR_CUDA, (st, nat.last_error())
 lib.msc_plan_destroy(h)
-''', tmp_path, FAKE_CUDA_FAIL=kernel, MSC_TUNE="c64=0,c32=0,bi=128")
+''', FAKE_CUDA_FAIL=kernel, MSC_TUNE="c64=0,c32=0,bi=128")
 
 
 @pytest.mark.parametrize("made", sorted({m for _, m in CASES}))
-def test_without_a_failure_the_solve_succeeds(made, tmp_path):
+def test_without_a_failure_the_solve_succeeds(made):
     fake_cuda.run(f'''
 h = {made}
 res = nat.Result()
 assert lib.msc_solve(h, None, None, ctypes.byref(res), side) == 0, nat.last_error()
 lib.msc_plan_destroy(h)
-''', tmp_path, MSC_TUNE="c64=0,c32=0,bi=128")
+''', MSC_TUNE="c64=0,c32=0,bi=128")

@@ -14,7 +14,7 @@ from . import fake_cuda
 
 @pytest.mark.parametrize("mixed", [False, True])
 @pytest.mark.parametrize("n", [30, 33])
-def test_autotuner_waits_for_the_box_lists(mixed, n, tmp_path):
+def test_autotuner_waits_for_the_box_lists(mixed, n):
     fake_cuda.run(f'''
 h = plan({n}, 9, separable=True, mixed={mixed})
 res = nat.Result()
@@ -22,12 +22,12 @@ lib.msc_solve(h, None, None, ctypes.byref(res), side)
 assert any("k_coupling_box" in x for x in report("launch"))
 assert report("unordered") == [], report("unordered")
 lib.msc_plan_destroy(h)
-''', tmp_path)
+''')
 
 
 @pytest.mark.parametrize("call", ["msc_solve_lower_block", "msc_apply_lower_block"])
 @pytest.mark.parametrize("solved_before", [False, True])
-def test_lower_block_waits_for_its_tables(call, solved_before, tmp_path):
+def test_lower_block_waits_for_its_tables(call, solved_before):
     # on a plan that was not made for Gauss-Seidel: the level tables are built by this call
     fake_cuda.run(f'''
 h = plan(30, 9, separable=False)
@@ -37,4 +37,4 @@ if {solved_before}:
 assert lib.{call}(h, buf(h), buf(h), side) == 0
 assert report("unordered") == [], report("unordered")
 lib.msc_plan_destroy(h)
-''', tmp_path)
+''')
