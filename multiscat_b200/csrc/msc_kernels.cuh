@@ -2130,14 +2130,38 @@ k_gradient_planes(int nkx, int nky, int n, int nsys, const int *__restrict__ pos
     for (int s = 0; s < nsys; ++s) {
         const int *map = pos_map + (size_t)s * ntor;
         if (s > 0) __syncthreads();
+        bool odd = false;
         for (int i = threadIdx.x; i < ntor; i += blockDim.x) {
             const int r = __ldg(map + i), x = i / nky, y = i - x * nky;
-            const double2 zero = make_double2(0.0, 0.0);
-            Ls[x * ld + y] = r >= 0 ? lam[(size_t)r * n + z] : zero;
-            Ps[x * ld + y] = r >= 0 ? psi[(size_t)r * n + z] : zero;
+            double2 l = make_double2(0.0, 0.0), q = l;
+            if (r >= 0) {
+                l = lam[(size_t)r * n + z];
+                q = psi[(size_t)r * n + z];
+            }
+            Ls[x * ld + y] = l;
+            Ps[x * ld + y] = q;
+            odd |= !isfinite(l.x) || !isfinite(l.y) || !isfinite(q.x) || !isfinite(q.y);
         }
-        __syncthreads();
+        odd = __syncthreads_or(odd);
         if (!work) continue;
+        if (odd) {
+            // infinities or NaN (a system that diverged): the zeros of absent channels
+            // must not meet them, so only pairs of channels are summed
+            for (int g = 0; g < ntor; ++g) {
+                if (__ldg(map + g) < 0) continue;
+                const int gx = g / nky, gy = g - gx * nky, sx = gx - dx + (gx < dx ? nkx : 0);
+                const double2 l = Ls[gx * ld + gy];
+#pragma unroll
+                for (int k = 0; k < KD; ++k) {
+                    const int sy = ((gy - dy0 - k) % nky + nky) % nky;
+                    if (__ldg(map + sx * nky + sy) < 0) continue;
+                    const double2 q = Ps[sx * ld + sy];
+                    acc[k].x = fma(l.x, q.x, fma(l.y, q.y, acc[k].x));
+                    acc[k].y = fma(l.x, q.y, fma(-l.y, q.x, acc[k].y));
+                }
+            }
+            continue;
+        }
         for (int gx = 0; gx < nkx; ++gx) {
             const double2 *lrow = Ls + gx * ld;
             const double2 *prow = Ps + (gx - dx + (gx < dx ? nkx : 0)) * ld;
