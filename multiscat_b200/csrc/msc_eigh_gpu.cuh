@@ -45,6 +45,8 @@ constexpr int kTriSmemMaxN = 160;          // n^2 doubles in one CTA's shared me
 //   v^T S v = inv^2 (x^T y - 2 alpha y_0 + alpha^2 S_00)
 // so that the product with S needs x only and runs before the norm is known.  alpha
 // has the sign opposite to x_0: nothing cancels in x_0 - alpha or y - alpha s0.
+// (x^T y and the terms beside it are of third order in the matrix: the caller keeps its
+// largest entry between 2^-200 and 2^200 by a power of two.)
 struct TriStep {
     double alpha, inv, vp;
     bool applied;
@@ -65,7 +67,7 @@ __device__ __forceinline__ TriStep tri_step(int m, const double *x, const double
         const double x0 = x[0];
         t.alpha = (x0 >= 0.0) ? -sqrt(n2) : sqrt(n2);
         t.inv = 1.0 / sqrt(n2 - x0 * x0 + (x0 - t.alpha) * (x0 - t.alpha));
-        t.vp = t.inv * t.inv * (xy - 2.0 * t.alpha * y[0] + t.alpha * t.alpha * s0[0]);
+        t.vp = t.inv * (t.inv * (xy - 2.0 * t.alpha * y[0] + t.alpha * t.alpha * s0[0]));
     }
     return t;
 }

@@ -2223,6 +2223,15 @@ msc_status device_symmetric_eigh(int n, const double *H, double *w, double *E)
     DevBuf<int4> groups;
     DevBuf<double2> tab;
     std::vector<double> Hh(H, H + (size_t)n * n);
+    // far from 1 the matrix is scaled by a power of two (no significand changes), so
+    // that the reduction's third-order products stay in range
+    double largest = 0.0;
+    for (double h : Hh) largest = std::max(largest, std::fabs(h));
+    int scale = 0;
+    if (largest > 0.0 && std::isfinite(largest) && std::abs(std::ilogb(largest)) > 200) {
+        scale = std::ilogb(largest);
+        for (double &h : Hh) h = std::ldexp(h, -scale);
+    }
     MSC_CUDA(upload(A, Hh));
     MSC_CUDA(R.alloc((size_t)n * n));
     MSC_CUDA(d.alloc(n));
@@ -2332,7 +2341,7 @@ msc_status device_symmetric_eigh(int n, const double *H, double *w, double *E)
     std::stable_sort(order.begin(), order.end(), [&](int i, int j) { return dh[i] < dh[j]; });
     for (int k = 0; k < n; ++k) {
         desth[order[k]] = k;
-        w[k] = dh[order[k]];
+        w[k] = std::ldexp(dh[order[k]], scale);
     }
     MSC_CUDA(upload(dest, desth));
     MSC_CUDA(Ed.alloc((size_t)n * n));
