@@ -2102,6 +2102,27 @@ k_potential_gradient(int nkx, int nky, int n, int nsys, const int *__restrict__ 
     }
 }
 
+// One offset's sum over pairs of channels, from the planes of k_gradient_planes: for a
+// system with infinities or NaN (it diverged), which the zeros of absent channels must
+// not meet.
+__device__ __noinline__ double2 gradient_pairs(int nkx, int nky, const int *__restrict__ map, const double2 *Ls,
+                                               const double2 *Ps, int dx, int dy)
+{
+    const int ld = nky | 1;
+    double2 acc = make_double2(0.0, 0.0);
+    for (int gx = 0; gx < nkx; ++gx) {
+        const int sx = gx - dx + (gx < dx ? nkx : 0);
+        for (int gy = 0; gy < nky; ++gy) {
+            const int sy = gy - dy + (gy < dy ? nky : 0);
+            if (__ldg(map + gx * nky + gy) < 0 || __ldg(map + sx * nky + sy) < 0) continue;
+            const double2 l = Ls[gx * ld + gy], q = Ps[sx * ld + sy];
+            acc.x = fma(l.x, q.x, fma(l.y, q.y, acc.x));
+            acc.y = fma(l.x, q.y, fma(-l.y, q.x, acc.y));
+        }
+    }
+    return acc;
+}
+
 // The same sums from shared memory: a block takes one z, stages lambda and psi of one
 // system at a time on their channel torus (absent channels zero), and each thread sums
 // KD neighbouring y offsets of one x offset.  Along a row the KD psi values a lambda
@@ -2145,21 +2166,9 @@ k_gradient_planes(int nkx, int nky, int n, int nsys, const int *__restrict__ pos
         odd = __syncthreads_or(odd);
         if (!work) continue;
         if (odd) {
-            // infinities or NaN (a system that diverged): the zeros of absent channels
-            // must not meet them, so only pairs of channels are summed
-            for (int g = 0; g < ntor; ++g) {
-                if (__ldg(map + g) < 0) continue;
-                const int gx = g / nky, gy = g - gx * nky, sx = gx - dx + (gx < dx ? nkx : 0);
-                const double2 l = Ls[gx * ld + gy];
 #pragma unroll
-                for (int k = 0; k < KD; ++k) {
-                    const int sy = ((gy - dy0 - k) % nky + nky) % nky;
-                    if (__ldg(map + sx * nky + sy) < 0) continue;
-                    const double2 q = Ps[sx * ld + sy];
-                    acc[k].x = fma(l.x, q.x, fma(l.y, q.y, acc[k].x));
-                    acc[k].y = fma(l.x, q.y, fma(-l.y, q.x, acc[k].y));
-                }
-            }
+            for (int k = 0; k < KD; ++k)
+                acc[k] = cadd(acc[k], gradient_pairs(nkx, nky, map, Ls, Ps, dx, (dy0 + k) % nky));
             continue;
         }
         for (int gx = 0; gx < nkx; ++gx) {
