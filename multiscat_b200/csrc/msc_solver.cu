@@ -994,9 +994,11 @@ template <> C2<double> *precond_term<double>(msc_plan *p) { return p->T64.p; }
 // Mixed form: the inner solve of a refinement step stops at this part of the tolerance.
 // Its estimate (FP32, BF16x3 inverse) is a little below the true residual; stopped at the
 // tolerance itself, a system that just misses it pays another refinement step, and the
-// others end right at it: half leaves residuals as with an FP32 inverse (81 x 81 x 300:
-// 1.6e-13 -> 1.0e-13 at 2e-13, refinement steps 4.5 -> 4.0 on average) for about one
-// more inner step (512 beams 50.9 -> 51.7 ms).
+// others end right at it.  Half brings psi nearer to 64 bits (512 beams, worse of two
+// inputs, 1.5e-10 -> 3.3e-11; 81 x 81 x 300, median of 32, 4.9e-12 -> 3.2e-12) for about one
+// more inner step (512 beams 50.9 -> 51.7 ms).  The Gauss-Seidel form keeps the tolerance:
+// its sweep is FP32 throughout and a step costs 50 block inverses (21 x 21 x 150, order 1:
+// 214 ms a solve, 226 with one more step).
 constexpr double kInnerMargin = 0.5;
 
 template <typename R>
@@ -1005,7 +1007,7 @@ void record_iterations_t(msc_plan *p, C2<R> *Q, C2<R> *W, C2<R> *U, cudaStream_t
     const size_t vs = (size_t)p->R * p->n;
     const bool tm = p->timing;
     const double inner = p->mixed ? p->inner_rtol : 0.0;
-    const double target = p->mixed ? kInnerMargin * p->desc.rtol : p->desc.rtol;
+    const double target = p->mixed && !p->gs ? kInnerMargin * p->desc.rtol : p->desc.rtol;
     for (int j = 0; j < p->m; ++j) {
         C2<R> *Qj = Q + (size_t)j * vs;
         C2<R> *Qn = Q + (size_t)(j + 1) * vs;
