@@ -66,7 +66,9 @@ typedef struct {
     int32_t max_refinements;/* mixed: outer FP64 refinement steps (0 = 30)      */
     int32_t flags;          /* bit 0: mixed form without the tcgen05 kernel;
                                bit 1: keep the tcgen05 kernel even when the
-                               autotuner times the SIMT kernel faster;
+                               autotuner times the SIMT kernel faster, and
+                               use it for 225 to 560 nodes too, where plans
+                               without this bit keep FP32 products;
                                bit 2: mixed form with ONE Gram-Schmidt pass
                                (Pythagorean norm) in the inner solve instead
                                of two; fewer bytes per iteration, but on
@@ -80,7 +82,11 @@ typedef struct {
                                bit 5: block Gauss-Seidel preconditioner, the
                                reference's: L = D + V^lower in each system's
                                channel order, M = L^-1 by a forward sweep
-                               (multiscat_gmres.f90:641-687)                  */
+                               (multiscat_gmres.f90:641-687);
+                               bit 6: the plan is for one solve: a short FP64
+                               solve then runs without recording a CUDA graph
+                               (plans without it record theirs in their first
+                               call and never later)                          */
     int32_t precond_order;  /* order k of the preconditioner series
                                M = sum_{i<=k} (-B^-1 N)^i B^-1 with B = D,
                                N = V (von Neumann, the reference's

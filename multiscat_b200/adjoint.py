@@ -24,7 +24,7 @@ class _ScatteringIntensities(torch.autograd.Function):
     @staticmethod
     def forward(ctx, potential: torch.Tensor, kinetic, systems, plan_kwargs, window):
         v = potential.detach().to("cpu", torch.complex128).numpy()
-        plan = ScatteringPlan(v, kinetic, systems, **plan_kwargs)
+        plan = ScatteringPlan(v, kinetic, systems, **{"_single_use": True, **plan_kwargs})
         res = plan.solve()
         ctx.plan = plan
         ctx.window = window

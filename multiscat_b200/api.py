@@ -333,7 +333,8 @@ def _single_solve(condition: ScatteringCondition, config: OptimizationConfig, *,
     plan = ScatteringPlan(arr.potential_values, arr.kinetic, [system],
                           rtol=config.residual_tolerance, restart=config.restart,
                           max_iterations=config.max_iterations,
-                          precision=config.precision_mode, preconditioner_order=order)
+                          precision=config.precision_mode, preconditioner_order=order,
+                          _single_use=True)
     try:
         result = plan.solve(raise_on_error=False)
     finally:
@@ -392,7 +393,8 @@ def get_scattering_state(condition: ScatteringCondition, config: OptimizationCon
     nkx, nky, nz = arr.potential_values.shape
     plan = ScatteringPlan(arr.potential_values, arr.kinetic, [system],
                           rtol=config.residual_tolerance, restart=config.restart,
-                          max_iterations=config.max_iterations, precision=config.precision_mode)
+                          max_iterations=config.max_iterations, precision=config.precision_mode,
+                          _single_use=True)
     try:
         if initial_state is not None:
             guess = np.asarray(initial_state, np.complex128).reshape(nkx, nky, nz)
@@ -429,7 +431,8 @@ def get_scattering_matrix_from_state(state: np.ndarray, condition: ScatteringCon
     grid = np.asarray(state, np.complex128).reshape(nkx, nky, nz)
     if convention == "reference":
         system = _reference_order_system(arr, n_channels)
-        plan = ScatteringPlan(arr.potential_values, arr.kinetic, [system], restart=1)
+        plan = ScatteringPlan(arr.potential_values, arr.kinetic, [system], restart=1,
+                              _single_use=True)
         try:
             rows = torch.as_tensor(np.ascontiguousarray(grid[system.channel_ix, system.channel_iy]),
                                    device=torch.device("cuda", torch.cuda.current_device()))
@@ -454,7 +457,7 @@ def get_scattering_matrices(conditions: Sequence[ScatteringCondition],
     plan = ScatteringPlan(grid.potential_values, grid.kinetic, systems,
                           rtol=config.residual_tolerance, restart=config.restart,
                           max_iterations=config.max_iterations,
-                          precision=config.precision_mode)
+                          precision=config.precision_mode, _single_use=True)
     try:
         result = plan.solve(raise_on_error=False)
     finally:

@@ -355,7 +355,6 @@ struct msc_plan {
     int cycles_last = 0;
     int fallbacks_last = 0;              // systems re-solved in FP64 by the last msc_solve
     int64_t launches_cycle = 0;          // kernel nodes of the cycle graph
-    int solves = 0;                      // msc_solve calls so far
     cudaError_t launch_error = cudaSuccess;   // first failed launch since the last check
 
     ~msc_plan()
@@ -473,6 +472,8 @@ using C2 = typename msc::CT<R>::t;
 
 template <typename R>
 size_t smem_block_inverse_t(int n) { return (size_t)2 * n * 2 * block_inverse_rows(n) * sizeof(R); }
+
+constexpr int kSingleUse = 64;      // msc_plan_desc flag: the plan solves once
 
 // tc_groups code of the channel-major tcgen05 kernel (k_block_inverse_tcc)
 constexpr int kTcChannelMajor = 3;
@@ -1556,7 +1557,7 @@ msc_status autotune(msc_plan *p)
 {
     if (tune_from_env(p)) return MSC_OK;
     const TuneKey key{p->n, p->R, p->K, p->nkx, p->nky, p->B, p->mixed ? 1 : 0, p->halo_hx,
-                      p->halo_hy, p->use_tc ? p->tc_n : 0, p->desc.flags, p->sep_ok ? 1 : 0};
+                      p->halo_hy, p->use_tc ? p->tc_n : 0, p->desc.flags & ~kSingleUse, p->sep_ok ? 1 : 0};
     {
         std::lock_guard<std::mutex> lock(g_tune_mutex);
         auto it = g_tune_cache.find(key);
@@ -2130,6 +2131,12 @@ msc_status finalize(msc_plan *p)
     for (int s = 0; s < p->B; ++s) p->kcyc_host[s] = 0;
     MSC_CUDA(p->report.alloc(p->B + 1));
     MSC_CUDA(cudaStreamSynchronize(0));      // everything above is in place for the plan's stream
+    // A kept plan records its graph here, in its first call, and never later: while a
+    // thread records, device-wide waits of other threads fail.
+    if (!(p->desc.flags & kSingleUse)) {
+        msc_status cst = capture(p, record_cycle, &p->g_cycle, &p->launches_cycle);
+        if (cst != MSC_OK) return cst;
+    }
     p->finalized = true;
     return MSC_OK;
 }
@@ -2405,7 +2412,7 @@ msc_status fp64_recover(msc_plan *p, const std::vector<int> &failed, const std::
     msc_plan_desc d = p->desc;
     d.precision = MSC_PRECISION_FP64;
     d.n_systems = nf;
-    d.flags = 0;
+    d.flags = kSingleUse;
     msc_plan *c = nullptr;
     msc_status st = msc_plan_create(&c, &d);
     if (st != MSC_OK) return st;
@@ -2765,16 +2772,14 @@ msc_status msc_solve(msc_plan *p, double *psi_out, double *intensities_out, msc_
         live = *p->counter_host != 0;
     }
     int cycle = 0;
-    // A plan's first two solves run up to two FP64 cycles as plain launches: a one-shot
-    // call never pays for the graph (0.3 to 0.5 ms to record, build and destroy), and
-    // its kernels take longer than their launches.  Longer solves, later ones and the
-    // mixed form (three or more cycles, whose last steps are launches of systems that
-    // stopped: 2 us each, less than a plain launch takes) use one graph per cycle.
-    // Measured, ms, graph / plain: 11 x 11 x 100 2.6 / 2.3, 7 x 5 x 81 1.8 / 1.7; mixed
-    // forward and backward 41 x 41 x 200 12.4 / 13.5.
-    ++p->solves;
+    // A plan for one solve runs up to two FP64 cycles as plain launches: such a call never
+    // pays for the graph (0.3 to 0.5 ms to record, build and destroy), and its kernels take
+    // longer than their launches.  Longer solves and the mixed form (three or more cycles,
+    // whose last steps are launches of systems that stopped: 2 us each, less than a plain
+    // launch takes) use one graph per cycle.  Measured, ms, graph / plain: 11 x 11 x 100 2.6
+    // / 2.3, 7 x 5 x 81 1.8 / 1.7; mixed forward and backward 41 x 41 x 200 12.4 / 13.5.
     for (; live && cycle < max_cycles; ++cycle) {
-        if (!p->g_cycle && (p->mixed || p->solves > 2 || cycle >= 2)) {
+        if (!p->g_cycle && (p->mixed || cycle >= 2)) {
             st = capture(p, record_cycle, &p->g_cycle, &p->launches_cycle);
             if (st != MSC_OK) return st;
         }
@@ -3244,6 +3249,7 @@ int msc_run_multiscat(int gmres_preconditioner_flag, int convergence_significant
     d.max_iterations = 2000;
     d.rtol = 5e-4 * std::pow(10.0, -(double)convergence_significant_figures);
     d.precision = MSC_PRECISION_FP64;
+    d.flags = kSingleUse;
     msc_plan *p = nullptr;
     msc_status st = msc_plan_create(&p, &d);
     if (st != MSC_OK) return st;

@@ -129,7 +129,7 @@ class ScatteringPlan:
                  max_refinements: int = 0, tensor_cores: bool | None = None,
                  inner_gram_schmidt_passes: int = 2, preconditioner_order: int = 0,
                  fp64_recovery: bool = True, gram_schmidt: str = "dcgs2",
-                 gauss_seidel: bool = False):
+                 gauss_seidel: bool = False, _single_use: bool = False):
         self._lib = nat.load()
         v = np.ascontiguousarray(np.asarray(potential_values), dtype=np.complex128)
         nkx, nky, nz = v.shape
@@ -170,6 +170,9 @@ class ScatteringPlan:
         # block-diagonal D^-1 series
         if gauss_seidel:
             desc.flags |= 32
+        # the package's own calls that make a plan for one solve: no graph for a short one
+        if _single_use:
+            desc.flags |= 64
         # von Neumann order k: M = sum_{i<=k} (-D^-1 V)^i D^-1 (0 = block-diagonal D^-1)
         desc.precond_order = int(preconditioner_order)
         self._plan = ctypes.c_void_p()

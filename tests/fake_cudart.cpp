@@ -4,7 +4,8 @@
 //    fills, kernels) may still be under way: no host wait and no event orders them
 //    (a copy to the device from pageable memory may return before it has arrived);
 //  - kernels in launch order, and fails the launches whose name holds FAKE_CUDA_FAIL.
-// fake_report() returns one line per event: "unordered NAME", "launch NAME" or "grid X Y NAME".
+// fake_report() returns one line per event: "unordered NAME", "launch NAME", "grid X Y
+// NAME" or "capture begin".
 // FAKE_CUDA_SMS: the device's SM count (148).
 #include <cuda_runtime_api.h>
 
@@ -143,7 +144,12 @@ cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned)
     stream_waited[s] = std::max(stream_waited[s], event_at[e]);
     return cudaSuccess;
 }
-cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { capturing = true; return cudaSuccess; }
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode)
+{
+    capturing = true;
+    report += "capture begin\n";
+    return cudaSuccess;
+}
 cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t *g) { capturing = false; *g = static_cast<cudaGraph_t>(handle()); return cudaSuccess; }
 cudaError_t cudaGraphInstantiate(cudaGraphExec_t *e, cudaGraph_t, unsigned long long) { *e = static_cast<cudaGraphExec_t>(handle()); return cudaSuccess; }
 cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaSuccess; }
