@@ -158,12 +158,16 @@ def oracle_fixture_error(res, workload: str, beams: int, world: int) -> dict | N
 # of a kernel kind over the given number of channel rows, from the captures
 # summarised in profiles/ (file named beside each entry).  Used as the
 # `traffic` of a kernel's roofline line, scaled to the rows of an average
-# launch of this run.
+# launch of this run.  Captured on batches whose FP32 vector (rows x 150 x 8
+# bytes) is larger than the 126 MB L2: a smaller one's output stays in L2 and
+# its input may come from there.  (Of a 144 MB output the last 27 to 45 MB are
+# still in L2 when the launch ends, so the figures lie a little below the
+# algorithmic bytes.)
 NCU_TRAFFIC = {
     # (workload, kind): (bytes, rows of the captured launch, profile)
     ("cfg2", "coupling"): (439.8e6 + 138.9e6, 119741, "k_coupling_halo_f32_cfg2.md"),
-    ("cfg2", "coupling_sep"): (72.381e6 + 11.869e6, 30011, "arnoldi_step_boxes_tcc_128beams.md"),
-    ("cfg2", "block_inverse"): (37.017e6 + 2.097e6, 30011, "arnoldi_step_boxes_tcc_128beams.md"),
+    ("cfg2", "coupling_sep"): (288.58e6 + 116.78e6, 119741, "dram_boxes_tcc_512beams.md"),
+    ("cfg2", "block_inverse"): (147.21e6 + 98.95e6, 119741, "dram_boxes_tcc_512beams.md"),
 }
 
 
