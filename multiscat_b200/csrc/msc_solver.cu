@@ -2833,6 +2833,9 @@ msc_status msc_solve(msc_plan *p, double *psi_out, double *intensities_out, msc_
         status[s] = r.unfinished ? (int)MSC_ERR_NOT_CONVERGED : r.status;
         resid[s] = r.resid;
     }
+    // from a zero guess the first cycle is launched unseen; with zero right-hand sides it
+    // had nothing to do
+    if (std::all_of(cycles.begin(), cycles.end(), [](int k) { return k == 0; })) p->cycles_last = 0;
     p->fallbacks_last = 0;
     if (p->mixed && !(p->desc.flags & 8)) {
         std::vector<int> failed;
