@@ -1398,7 +1398,7 @@ msc_status setup_tensor_core(msc_plan *p)
     // Above 224 nodes the inner solve keeps FP32 products unless the caller asks for
     // tcgen05 (flag 2): against 64 bits a BF16x3 block inverse is 6.1e-6 to 7.0e-6 off
     // (2-norm), the FP32 one 4.6e-7 to 4.8e-7, and on 4 x 81 x 81 x 300 over 32 inputs
-    // psi was up to 3 times as far off as with FP32 products (97 ms a solve, 49 with it).
+    // psi was up to 4.6 times as far off as with FP32 products (97 ms a solve, 49 with it).
     if (chosen == 0) return (p->desc.flags & 2) ? setup_tc_stream(p, sms, (size_t)optin) : MSC_OK;
     p->tc_n = chosen;
     p->tc_groups = 1;
