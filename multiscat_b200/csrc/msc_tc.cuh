@@ -609,6 +609,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tc(TcParams prm)
             const uint32_t lanes = (uint32_t)(lq * 32) << 16;
 #pragma unroll
             for (int c0 = c_begin; c0 < c_begin + CW; c0 += 16) {
+                __syncwarp();                  // lanes past kp left the last pass early
                 uint32_t r[16], w[8];
                 if (some) {
                     tmem_ld16_nowait(tmem + lanes + (uint32_t)(m * N + c0), r);

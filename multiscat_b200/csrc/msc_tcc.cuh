@@ -400,6 +400,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_block_inverse_tcc(TcParams prm)
         float2 *urow = raw + (size_t)jc * n;
 #pragma unroll 1
         for (int u = 0; u < nu; ++u) {
+            __syncwarp();                      // lanes past the tile's rows left the last pass early
             uint32_t r[8];
             tmem_ld8_nowait(t2 + (uint32_t)(8 * u), r);
             tmem_wait_ld();
